@@ -52,6 +52,7 @@ SIGNATURES = {
                                           _ip, _dp, _dp, _dp],
     "f3d_ads_output_species": [_vp, _ip, C.c_int, _dp, _dp, _dp, _dp],
     "f3d_ads_set_meteo_corners": [_vp] + [_dp] * 6 + [C.c_double] * 4,
+    "f3d_ads_set_meteo_pairs_kdiffu": [_vp] + [_dp] * 12 + [C.POINTER(F3DKdiffu), C.c_double, C.c_double],
     "f3d_ads_set_meteo_corners_kdiffu": [_vp] + [_dp] * 8 + [C.POINTER(F3DKdiffu), C.c_double, C.c_double],
     "f3d_ads_set_source": [_vp, C.c_int, _ip, _dp],
     "f3d_ads_set_source_dense": [_vp, _dp],

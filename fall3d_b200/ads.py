@@ -119,9 +119,18 @@ class Domain:
         points (nx, ny)."""
         g = self.grid
 
+        keep = []
+
         def pair(p):
-            return None if p is None else np.asfortranarray(
-                np.stack([np.asarray(p[0], np.float64), np.asarray(p[1], np.float64)], axis=3))
+            """Pointers to the two time levels (arrays already in the reference's layout are not copied)."""
+            if p is None:
+                return None, None
+            lev = [np.asarray(p[0], np.float64), np.asarray(p[1], np.float64)]
+            if lev[0].shape != lev[1].shape or lev[0].ndim != 3:
+                both = np.asfortranarray(np.stack(lev, axis=3))
+                lev = [both[:, :, :, 0], both[:, :, :, 1]]
+            keep.extend(np.asfortranarray(a) for a in lev)
+            return _p(keep[-2]), _p(keep[-1])
         uc, vc, wc, tvc = pair(uc_pair), pair(vc_pair), pair(wc_pair), pair(tvc_pair)
         two = [None if a is None else np.asfortranarray(a, dtype=np.float64) for a in (pblh, mon, ust)]
         hc = np.asfortranarray(g.h_c, dtype=np.float64) if modkv == 3 else None
@@ -129,10 +138,9 @@ class Domain:
             self._ensure_corner_heights()
         kd = F3DKdiffu(int(modkh), int(modkv), int(g.map_h), float(kh0), float(kv0), float(rams_cs),
                        float(g.dlon), float(g.dlat), float(s_time))
-        check(lib().f3d_ads_set_meteo_corners_kdiffu(self._h, _p(uc), _p(vc), _p(wc), _p(tvc),
-                                                     *[_p(a) for a in two], _p(hc), C.byref(kd),
-                                                     float(t_its), float(t_ite)),
-              "f3d_ads_set_meteo_corners_kdiffu")
+        check(lib().f3d_ads_set_meteo_pairs_kdiffu(self._h, *uc, *vc, *wc, *tvc, *[_p(a) for a in two], _p(hc),
+                                                   C.byref(kd), float(t_its), float(t_ite)),
+              "f3d_ads_set_meteo_pairs_kdiffu")
 
     def phys_wet_deposition(self, a, b, pre, pblh, bin_cat, bin_diam):
         """Switch on wet deposition for this meteo interval (precipitation

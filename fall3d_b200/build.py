@@ -29,6 +29,7 @@ SOURCES = [
     ("meteo_dev.cu", ["--fmad=false"]),
     ("deposit_dev.cu", ["--fmad=false"]),
     ("output_dev.cu", ["--fmad=false"]),
+    ("state_io.cu", []),
     ("f3d_capi.cu", ["-Xcompiler", "-ffp-contract=off"]),
 ]
 

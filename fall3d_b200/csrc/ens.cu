@@ -20,6 +20,7 @@
 #include "f3d_common.cuh"
 #include "phys_dev.cuh"
 #include "phys_host.h"
+#include "state_io.h"
 #include "step_dev.cuh"
 
 namespace f3d {
@@ -164,6 +165,7 @@ struct f3d_ens {
   size_t staging_elems = 0;
   double* h_pin = nullptr;
   size_t h_pin_elems = 0;
+  StateIO io;  // transfers of the members' host arrays
   int iiter = 0;
   bool dm_valid = false;  // the device member table has been written once
   cudaGraphExec_t graph[2] = {nullptr, nullptr};
@@ -319,6 +321,7 @@ extern "C" int f3d_ens_destroy(f3d_ens* e) {
   cudaSetDevice(e->device);
   if (e->st) cudaStreamSynchronize(e->st);
   drop_graphs(e);
+  e->io.release();
   for (void* p : e->work_allocs) cudaFree(p);
   for (void* p : e->allocs) cudaFree(p);
   if (e->d_met) cudaFree(e->d_met);
@@ -891,28 +894,11 @@ extern "C" int f3d_ens_upload_member_state(f3d_ens* e, int mi, const double* my_
 extern "C" int f3d_ens_download_member_state(f3d_ens* e, int mi, double* my_c, double* my_acum) {
   if (!e || mi < 0 || mi >= e->nm) return set_error_msg("f3d_ens_download_member_state: bad member");
   ECK(cudaSetDevice(e->device));
-  ECK(cudaStreamSynchronize(e->st));
   const EnsClass& k = e->cls[e->member_class[mi]];
   const MemberDev& m = e->hm[mi];
-  const size_t nx = k.nx, ny = k.ny, nz = k.nz, nb = e->nb;
+  const size_t nx = k.nx, ny = k.ny, nb = e->nb;
   if (my_c) {
-    std::vector<double> tmp(nx * ny * nz * nb);
-    if (e->prec == F3D_PREC_FP64) {
-      ECK(cudaMemcpy(tmp.data(), m.c64, tmp.size() * 8, cudaMemcpyDeviceToHost));
-    } else {
-      std::vector<float> t32(tmp.size());
-      ECK(cudaMemcpy(t32.data(), m.c32, t32.size() * 4, cudaMemcpyDeviceToHost));
-      for (size_t q = 0; q < t32.size(); ++q) tmp[q] = t32[q];
-      if (m.c32lo) {
-        ECK(cudaMemcpy(t32.data(), m.c32lo, t32.size() * 4, cudaMemcpyDeviceToHost));
-        for (size_t q = 0; q < t32.size(); ++q) tmp[q] = tmp[q] + (double)t32[q];
-      }
-    }
-    for (size_t b = 0; b < nb; ++b)
-      for (size_t kk = 0; kk < nz; ++kk)
-        for (size_t j = 0; j < ny; ++j)
-          memcpy(&my_c[2 + (nx + 4) * ((j + 2) + (ny + 4) * ((kk + 2) + (nz + 4) * b))],
-                 &tmp[((b * nz + kk) * ny + j) * nx], nx * 8);
+    ECK(e->io.download(rows3d(m, my_c, false), e->device, e->st));
     if (m.gh64 || m.gh32) {  // the kept boundary halo layers
       std::vector<double> g((size_t)gh_per_bin(m.nx, m.ny, m.nz) * nb);
       if (m.gh64) {
@@ -925,13 +911,8 @@ extern "C" int f3d_ens_download_member_state(f3d_ens* e, int mi, double* my_c, d
       gh_scatter_ref(m.nx, m.ny, m.nz, (int)nb, g, my_c);
     }
   }
-  if (my_acum) {
-    std::vector<double> tmp(nx * ny * nb);
-    ECK(cudaMemcpy(tmp.data(), m.acum, tmp.size() * 8, cudaMemcpyDeviceToHost));
-    for (size_t b = 0; b < nb; ++b)
-      for (size_t j = 0; j < ny; ++j)
-        memcpy(&my_acum[2 + (nx + 4) * ((j + 2) + (ny + 4) * b)], &tmp[(b * ny + j) * nx], nx * 8);
-  }
+  if (my_acum) ECK(e->io.download(rows2d(m.acum, nx, ny, nb, my_acum), e->device, e->st));
+  if (!my_c && !my_acum) ECK(cudaStreamSynchronize(e->st));
   return 0;
 }
 

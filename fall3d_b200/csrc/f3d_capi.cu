@@ -16,6 +16,7 @@
 #include "f3d_common.cuh"
 #include "phys_dev.cuh"
 #include "phys_host.h"
+#include "state_io.h"
 
 namespace f3d {
 // ads_fp64.cu
@@ -145,6 +146,7 @@ struct f3d_ctx {
   double* d_red = nullptr;    // reduction scratch (CFL 3 doubles, mass partials)
   int mass_nblk = 148 * 2;
   double* h_pin = nullptr;    // pinned host scratch (fluxes, reductions)
+  StateIO io;                 // transfers of the large host arrays
   int* d_nfail = nullptr;
   double t_its = 0.0, t_ite = 1.0;
   bool grid_set = false, meteo_set = false;
@@ -399,6 +401,7 @@ extern "C" int f3d_ads_destroy(f3d_ctx* c) {
   if (!c) return 0;
   cudaSetDevice(c->device);
   if (c->st) cudaStreamSynchronize(c->st);
+  c->io.release();
   for (void* p : c->allocs) cudaFree(p);
   if (c->d_rhoc_tc) cudaFree(c->d_rhoc_tc);
   if (c->h_pin) cudaFreeHost(c->h_pin);
@@ -549,17 +552,29 @@ extern "C" int f3d_ads_set_terrain(f3d_ctx* c, int map_v, double X3max, const do
   return 0;
 }
 
+// A corner field at the two time levels of a meteo interval: one array of
+// both, or two.
+struct Pair {
+  const double* s[2];
+  Pair(const double* both, size_t n) : s{both, both ? both + n : nullptr} {}
+  Pair(const double* a, const double* b) : s{a, b} {}
+  bool ok() const { return s[0] && s[1]; }
+};
+static size_t ncorners(const f3d_ctx* c) {
+  return c ? (size_t)(c->nx + 1) * (c->ny + 1) * (c->nz + 1) : 0;
+}
+
 // The meteo term from corner fields (F3D_update_meteo_term compute part):
 // uploads the corner winds of both snapshots, lets fill_k write the
 // unscaled diffusion into dk1..dk3 (reference layouts), then staggers and
 // scales on the device.
 template <class FillK>
-static int meteo_corners_impl(f3d_ctx* c, const char* who, const double* uc, const double* vc,
-                              const double* wc, size_t extra, double t_its, double t_ite,
+static int meteo_corners_impl(f3d_ctx* c, const char* who, const Pair& uc, const Pair& vc,
+                              const Pair& wc, size_t extra, double t_its, double t_ite,
                               FillK fill_k) {
   if (!c) return set_err("%s: null context", who);
   if (!c->grid_set) return set_err("%s: grid not set", who);
-  if (!uc || !vc || !wc) return set_err("%s: null corner wind", who);
+  if (!uc.ok() || !vc.ok() || !wc.ok()) return set_err("%s: null corner wind", who);
   if (!(t_ite != t_its)) return set_err("%s: t_ite == t_its", who);
   CK(cudaSetDevice(c->device));
   const size_t nx = c->nx, ny = c->ny, nz = c->nz;
@@ -578,9 +593,11 @@ static int meteo_corners_impl(f3d_ctx* c, const char* who, const double* uc, con
   double* dk2 = dk1 + n1;
   double* dk3 = dk2 + n2;
   double* dextra = dk3 + n3;
-  CK(cudaMemcpyAsync(duc, uc, 2 * ncor * 8, cudaMemcpyHostToDevice, c->st));
-  CK(cudaMemcpyAsync(dvc, vc, 2 * ncor * 8, cudaMemcpyHostToDevice, c->st));
-  CK(cudaMemcpyAsync(dwc, wc, 2 * ncor * 8, cudaMemcpyHostToDevice, c->st));
+  for (int q = 0; q < 2; ++q) {
+    CK(c->io.upload(duc + q * ncor, uc.s[q], ncor * 8, c->device, c->st));
+    CK(c->io.upload(dvc + q * ncor, vc.s[q], ncor * 8, c->device, c->st));
+    CK(c->io.upload(dwc + q * ncor, wc.s[q], ncor * 8, c->device, c->st));
+  }
   if (fill_k(duc, dvc, dk1, dk2, dk3, dextra)) return 1;
   MemberDev& m = c->hm;
   MetGeo g;
@@ -626,7 +643,8 @@ extern "C" int f3d_ads_set_meteo_corners(f3d_ctx* c, const double* uc, const dou
   if (kgiven && !(k1 && k2 && k3))
     return set_err("f3d_ads_set_meteo_corners: give all of k1, k2, k3 or none");
   return meteo_corners_impl(
-      c, "f3d_ads_set_meteo_corners", uc, vc, wc, 0, t_its, t_ite,
+      c, "f3d_ads_set_meteo_corners", Pair(uc, ncorners(c)), Pair(vc, ncorners(c)),
+      Pair(wc, ncorners(c)), 0, t_its, t_ite,
       [&](double*, double*, double* dk1, double* dk2, double* dk3, double*) -> int {
         const size_t nx = c->nx, ny = c->ny, nz = c->nz;
         if (kgiven) {
@@ -641,12 +659,9 @@ extern "C" int f3d_ads_set_meteo_corners(f3d_ctx* c, const double* uc, const dou
       });
 }
 
-extern "C" int f3d_ads_set_meteo_corners_kdiffu(f3d_ctx* c, const double* uc, const double* vc,
-                                                const double* wc, const double* tvc,
-                                                const double* pblh, const double* mon,
-                                                const double* ust, const double* h_c,
-                                                const f3d_kdiffu* kd, double t_its, double t_ite) {
-  const char* who = "f3d_ads_set_meteo_corners_kdiffu";
+static int meteo_kdiffu(f3d_ctx* c, const char* who, const Pair& uc, const Pair& vc, const Pair& wc,
+                        const Pair& tvc, const double* pblh, const double* mon, const double* ust,
+                        const double* h_c, const f3d_kdiffu* kd, double t_its, double t_ite) {
   if (!c || !kd) return set_err("%s: null argument", who);
   if (kd->modkh != 1 && kd->modkh != 2 && kd->modkh != 4)
     return set_err("Horizontal diffusion parameterization not implemented ");
@@ -655,7 +670,7 @@ extern "C" int f3d_ads_set_meteo_corners_kdiffu(f3d_ctx* c, const double* uc, co
   if (kd->map_h == 2 || kd->map_h == 3) return set_err("Mapping not implemented yet");
   if (kd->map_h != 0 && kd->map_h != 1) return set_err("Incorrect horizontal mapping");
   const bool vsim = kd->modkv == 3;
-  if (vsim && (!tvc || !pblh || !mon || !ust || !h_c))
+  if (vsim && (!tvc.ok() || !pblh || !mon || !ust || !h_c))
     return set_err("%s: the similarity K needs tvc, pblh, mon, ust and h_c", who);
   if (vsim && !c->d_zc)
     return set_err("%s: corner heights not set (f3d_ads_set_corner_heights)", who);
@@ -694,7 +709,8 @@ extern "C" int f3d_ads_set_meteo_corners_kdiffu(f3d_ctx* c, const double* uc, co
         a.zc = c->d_zc;
         double* p = dx;
         if (vsim) {
-          CK(cudaMemcpyAsync(p, tvc, 2 * ncor * 8, cudaMemcpyHostToDevice, c->st));
+          for (int q = 0; q < 2; ++q)
+            CK(c->io.upload(p + q * ncor, tvc.s[q], ncor * 8, c->device, c->st));
           a.tvc0 = p;
           a.tvc1 = p + ncor;
           p += 2 * ncor;
@@ -730,6 +746,26 @@ extern "C" int f3d_ads_set_meteo_corners_kdiffu(f3d_ctx* c, const double* uc, co
         c->launches += 2;
         return 0;
       });
+}
+
+extern "C" int f3d_ads_set_meteo_corners_kdiffu(f3d_ctx* c, const double* uc, const double* vc,
+                                                const double* wc, const double* tvc,
+                                                const double* pblh, const double* mon,
+                                                const double* ust, const double* h_c,
+                                                const f3d_kdiffu* kd, double t_its, double t_ite) {
+  const size_t n = ncorners(c);
+  return meteo_kdiffu(c, "f3d_ads_set_meteo_corners_kdiffu", Pair(uc, n), Pair(vc, n), Pair(wc, n),
+                      Pair(tvc, n), pblh, mon, ust, h_c, kd, t_its, t_ite);
+}
+
+extern "C" int f3d_ads_set_meteo_pairs_kdiffu(f3d_ctx* c, const double* uc0, const double* uc1,
+                                              const double* vc0, const double* vc1, const double* wc0,
+                                              const double* wc1, const double* tvc0, const double* tvc1,
+                                              const double* pblh, const double* mon,
+                                              const double* ust, const double* h_c,
+                                              const f3d_kdiffu* kd, double t_its, double t_ite) {
+  return meteo_kdiffu(c, "f3d_ads_set_meteo_pairs_kdiffu", Pair(uc0, uc1), Pair(vc0, vc1),
+                      Pair(wc0, wc1), Pair(tvc0, tvc1), pblh, mon, ust, h_c, kd, t_its, t_ite);
 }
 
 extern "C" int f3d_ads_set_wet_deposition(f3d_ctx* c, double a, double b, const double* pre,
@@ -788,18 +824,12 @@ extern "C" int f3d_ads_set_radionuclides(f3d_ctx* c, const int* bin_cat, const i
 extern "C" int f3d_ads_get_awet(f3d_ctx* c, double* my_awet) {
   if (!c || !my_awet) return set_err("f3d_ads_get_awet: null argument");
   const size_t nx = c->nx, ny = c->ny, nb = c->nb;
-  std::vector<double> d(nx * ny * nb, 0.0);
-  if (c->d_awet) {
-    CK(cudaSetDevice(c->device));
-    CK(cudaStreamSynchronize(c->st));
-    CK(cudaMemcpy(d.data(), c->d_awet, d.size() * 8, cudaMemcpyDeviceToHost));
-  }
   // my_awet(ips-2:ipe+2, jps-2:jpe+2, nbins), halos zero
   std::fill(my_awet, my_awet + (nx + 4) * (ny + 4) * nb, 0.0);
-  for (size_t b = 0; b < nb; ++b)
-    for (size_t j = 0; j < ny; ++j)
-      for (size_t i = 0; i < nx; ++i)
-        my_awet[(i + 2) + (nx + 4) * ((j + 2) + (ny + 4) * b)] = d[(b * ny + j) * nx + i];
+  if (c->d_awet) {
+    CK(cudaSetDevice(c->device));
+    CK(c->io.download(rows2d(c->d_awet, nx, ny, nb, my_awet), c->device, c->st));
+  }
   return 0;
 }
 
@@ -1105,53 +1135,12 @@ extern "C" int f3d_ads_upload_state(f3d_ctx* c, const double* my_c, const double
 extern "C" int f3d_ads_download_state(f3d_ctx* c, double* my_c, double* my_acum) {
   if (!c) return set_err("f3d_ads_download_state: null context");
   CK(cudaSetDevice(c->device));
-  CK(cudaStreamSynchronize(c->st));
   MemberDev& m = c->hm;
-  const size_t nx = c->nx, ny = c->ny, nz = c->nz, nb = c->nb;
+  const size_t nx = c->nx, ny = c->ny, nb = c->nb;
   if (my_c) {
-    std::vector<double> tmp(nx * ny * nz * nb);
-    if (c->prec == F3D_PREC_FP64) {
-      CK(cudaMemcpy(tmp.data(), m.c64, tmp.size() * 8, cudaMemcpyDeviceToHost));
-    } else {
-      std::vector<float> t32(tmp.size());
-      CK(cudaMemcpy(t32.data(), m.c32, t32.size() * 4, cudaMemcpyDeviceToHost));
-      for (size_t q = 0; q < t32.size(); ++q) tmp[q] = t32[q];
-      if (m.c32lo) {
-        CK(cudaMemcpy(t32.data(), m.c32lo, t32.size() * 4, cudaMemcpyDeviceToHost));
-        for (size_t q = 0; q < t32.size(); ++q) tmp[q] = tmp[q] + (double)t32[q];
-      }
-    }
-    const size_t X = nx + 4, Y = ny + 4, Z = nz + 4;
-    for (size_t b = 0; b < nb; ++b)
-      for (size_t k = 0; k < nz; ++k)
-        for (size_t j = 0; j < ny; ++j) {
-          const double* row = &tmp[((b * nz + k) * ny + j) * nx];
-          double* dst = &my_c[2 + X * ((j + 2) + Y * ((k + 2) + Z * b))];
-          memcpy(dst, row, nx * 8);
-          // zero-gradient face ghosts of the final state
-          dst[-1] = dst[-2] = row[0];
-          dst[nx] = dst[nx + 1] = row[nx - 1];
-        }
-    for (size_t b = 0; b < nb; ++b)
-      for (size_t k = 0; k < nz; ++k)
-        for (size_t i = 0; i < nx; ++i) {
-          double lo = tmp[((b * nz + k) * ny + 0) * nx + i];
-          double hi = tmp[((b * nz + k) * ny + (ny - 1)) * nx + i];
-          for (int g = 0; g < 2; ++g) {
-            my_c[(i + 2) + X * (g + Y * ((k + 2) + Z * b))] = lo;
-            my_c[(i + 2) + X * ((ny + 2 + g) + Y * ((k + 2) + Z * b))] = hi;
-          }
-        }
-    for (size_t b = 0; b < nb; ++b)
-      for (size_t j = 0; j < ny; ++j)
-        for (size_t i = 0; i < nx; ++i) {
-          double lo = tmp[((b * nz + 0) * ny + j) * nx + i];
-          double hi = tmp[((b * nz + (nz - 1)) * ny + j) * nx + i];
-          for (int g = 0; g < 2; ++g) {
-            my_c[(i + 2) + X * ((j + 2) + Y * (g + Z * b))] = lo;
-            my_c[(i + 2) + X * ((j + 2) + Y * ((nz + 2 + g) + Z * b))] = hi;
-          }
-        }
+    // the interior and the zero-gradient face ghosts of the final state; the
+    // halo's edges and corners stay as they are
+    CK(c->io.download(rows3d(m, my_c, true), c->device, c->st));
     if (m.gh64 || m.gh32) {  // the kept boundary halo layers replace the zero-gradient ghosts
       std::vector<double> g((size_t)gh_per_bin(c->nx, c->ny, c->nz) * nb);
       if (m.gh64) {
@@ -1164,13 +1153,8 @@ extern "C" int f3d_ads_download_state(f3d_ctx* c, double* my_c, double* my_acum)
       gh_scatter(c, g, my_c);
     }
   }
-  if (my_acum) {
-    std::vector<double> tmp(nx * ny * nb);
-    CK(cudaMemcpy(tmp.data(), m.acum, tmp.size() * 8, cudaMemcpyDeviceToHost));
-    for (size_t b = 0; b < nb; ++b)
-      for (size_t j = 0; j < ny; ++j)
-        memcpy(&my_acum[2 + (nx + 4) * ((j + 2) + (ny + 4) * b)], &tmp[(b * ny + j) * nx], nx * 8);
-  }
+  if (my_acum) CK(c->io.download(rows2d(m.acum, nx, ny, nb, my_acum), c->device, c->st));
+  if (!my_c && !my_acum) CK(cudaStreamSynchronize(c->st));
   return 0;
 }
 
@@ -1704,8 +1688,8 @@ static int stage_vset_inputs(f3d_ctx* c, const double* rhoc, const double* tc, c
     par[3 * b + 2] = psi[b];
     fl[b] = bin_cat[b] | ((is_aggregate && is_aggregate[b]) ? (1 << 8) : 0);
   }
-  CK(cudaMemcpyAsync(*drho, rhoc, ncor * 8, cudaMemcpyHostToDevice, c->st));
-  CK(cudaMemcpyAsync(*dt, tc, ncor * 8, cudaMemcpyHostToDevice, c->st));
+  CK(c->io.upload(*drho, rhoc, ncor * 8, c->device, c->st));
+  CK(c->io.upload(*dt, tc, ncor * 8, c->device, c->st));
   CK(cudaMemcpyAsync(*dpar, par.data(), par.size() * 8, cudaMemcpyHostToDevice, c->st));
   CK(cudaMemcpyAsync(*dflags, fl.data(), fl.size() * 4, cudaMemcpyHostToDevice, c->st));
   CK(cudaStreamSynchronize(c->st));
@@ -1723,7 +1707,9 @@ static int finish_vset(f3d_ctx* c, int nfail, double* vs_out) {
     if (n > c->staging_elems) return set_err("staging too small");
     launch_conv(9, c->hm.vs, c->staging, c->nx, c->ny, c->nz, c->nb, c->st);
     CKL();
-    CK(cudaMemcpyAsync(vs_out, c->staging, n * 8, cudaMemcpyDeviceToHost, c->st));
+    const long long nr = (long long)c->ny * (c->nz + 3) * c->nb;
+    CK(c->io.download(RowsOut{c->staging, nullptr, nullptr, c->nx, nr, 1, 1, vs_out, 0, c->nx, nr, 1, false},
+                      c->device, c->st));
   }
   CK(cudaStreamSynchronize(c->st));
   if (nfail) {

@@ -1,0 +1,61 @@
+// state_io.h -- host <-> device transfers of the large arrays.
+//
+// The reference arrays live in pageable host memory and hold FP64 values with
+// two halo cells around each plane; the device keeps interior cells in the
+// form it steps.  A StateIO moves them through a few page-locked slots: on
+// the way out a kernel writes the FP64 values of a range of rows straight
+// into a slot over PCIe, and a few host threads copy finished slots into the
+// caller's array while later ones fill.
+#pragma once
+#include <cuda_runtime.h>
+
+#include <cstddef>
+
+#include "f3d_common.cuh"
+
+namespace f3d {
+
+// Rows of a device array [b][k][j][i] and where they go in the host array:
+// row (b, k, j) starts at host[off + X * (j + Y * (k + Z * b))].  Exactly one
+// of c64, c32 is set; lo adds to c32 when given.
+struct RowsOut {
+  const double* c64;
+  const float* c32;
+  const float* lo;
+  long long nx, ny, nz, nb;
+  double* host;
+  long long off, X, Y, Z;
+  bool faces;  // also the zero-gradient face ghosts, two cells deep (needs the halo pitches)
+};
+
+// A member's concentration into my_c(ips-2:ipe+2, jps-2:jpe+2, kps-2:kpe+2, nbins).
+inline RowsOut rows3d(const MemberDev& m, double* my_c, bool faces) {
+  const long long X = m.nx + 4, Y = m.ny + 4, Z = m.nz + 4;
+  return RowsOut{m.c64, m.c32, m.c32lo, m.nx, m.ny, m.nz, m.nb, my_c, 2 + X * (2 + Y * 2), X, Y, Z, faces};
+}
+// A deposit [b][j][i] into my_acum(ips-2:ipe+2, jps-2:jpe+2, nbins).
+inline RowsOut rows2d(const double* a, long long nx, long long ny, long long nb, double* host) {
+  return RowsOut{a, nullptr, nullptr, nx, ny, 1, nb, host, 2 + (nx + 4) * 2, nx + 4, ny + 4, 1, false};
+}
+
+class StateIO {
+ public:
+  ~StateIO() { release(); }
+  // Both return cudaSuccess once the host array is complete (download) or the
+  // host array may change again (upload; the device side is complete too).
+  // Work already on the stream comes first.
+  cudaError_t download(const RowsOut& r, int device, cudaStream_t st);
+  cudaError_t upload(void* dst, const void* src, size_t bytes, int device, cudaStream_t st);
+  void release();
+
+ private:
+  static constexpr int kSlots = 8;             // two per host thread
+  static constexpr size_t kSlotBytes = 1 << 20;  // page-locking costs ~0.5 ms a MB, once
+  cudaError_t reserve(size_t total, size_t unit);
+  char* pin_ = nullptr;
+  size_t slot_bytes_ = 0;
+  int nslots_ = 0;
+  cudaEvent_t ev_[kSlots] = {};
+};
+
+}  // namespace f3d

@@ -162,6 +162,16 @@ int f3d_ads_set_meteo_corners_kdiffu(f3d_ctx *ctx, const double *uc,
                                      const double *mon, const double *ust,
                                      const double *h_c, const f3d_kdiffu *kd,
                                      double t_its, double t_ite);
+/* The same with the two time levels of each corner field in arrays of their
+ * own (tvc0 and tvc1 may be NULL where tvc may). */
+int f3d_ads_set_meteo_pairs_kdiffu(f3d_ctx *ctx, const double *uc0, const double *uc1,
+                                   const double *vc0, const double *vc1,
+                                   const double *wc0, const double *wc1,
+                                   const double *tvc0, const double *tvc1,
+                                   const double *pblh, const double *mon,
+                                   const double *ust, const double *h_c,
+                                   const f3d_kdiffu *kd, double t_its, double t_ite);
+
 
 /* Gravity current, F3D_add_radial_wind (mod_F3D.F90:978-1226).  params =
  * MY_MOD%MY_GC {lon, lat, start_time, end_time, c_flow_rate, k_entrain,

@@ -24,6 +24,7 @@
 #ifndef F3D_HALF_TAIL
 #define F3D_HALF_TAIL 1
 #endif
+#include "active.cuh"
 #include "march.cuh"
 #include "step_dev.cuh"
 
@@ -340,7 +341,8 @@ __device__ __forceinline__ void block_reduce2_f64(double a, double b, double* ou
 // so that the sweeps without it keep their register allocation.
 template <int DIR, int LIM, int TM, bool CMP = false, bool EPI = false>
 __device__ __forceinline__ void sweep32_item(const MemberDev* __restrict__ members,
-                                             const WorkItem w, int bpb, unsigned char* f3d_smem) {
+                                             const WorkItem w, int bpb,
+                                             const int2* __restrict__ ranges, unsigned char* f3d_smem) {
   const MemberDev& m = members[w.member];
   const int nx = m.nx, ny = m.ny, nz = m.nz;
   const long long nsp = (DIR == DIR_X) ? (long long)ny * nz
@@ -353,23 +355,32 @@ __device__ __forceinline__ void sweep32_item(const MemberDev* __restrict__ membe
   const bool run_it = (DIR == DIR_X) ? (pen0w < nsp && b < m.nb) : lane_ok;
   const long long pen = pen_raw < nsp ? pen_raw : nsp - 1;
   double clo = 0.0, chi = 0.0;
+  // the cells this sweep can change: positions 0..n-1 of the march are
+  // act.x..act.y-1 of the pencil (the epilogue counts levels: all of them)
+  int2 act = make_int2(0, (DIR == DIR_X) ? nx : (DIR == DIR_Y) ? ny : nz);
+  if (!EPI && ranges) act = __ldg(ranges + blockIdx.x);
+  if (act.x == act.y) {
+    if (lane_ok && m.gh32) {  // an empty pencil's ghosts
+      float* g = m.gh32 + (long long)b * gh_per_bin(nx, ny, nz);
+      g[gh_offset(DIR, 0, pen, nx, ny, nz)] = 0.f;
+      g[gh_offset(DIR, 1, pen, nx, ny, nz)] = 0.f;
+    }
+    if (threadIdx.x < 2) m.flux_part[2 * (long long)w.slot + threadIdx.x] = 0.0;
+    return;
+  }
   if (run_it) {
     Ops32<LIM, DIR, TM, CMP, EPI> o;
     double area;
-    int n, i = 0, j = 0;
+    const int lo = act.x, n = act.y - act.x;
+    int i = 0, j = 0;
     if (DIR == DIR_X) {
       j = (int)(pen % ny);
       int k = (int)(pen / ny);
-      n = nx;
       o.cp = m.c32 + (((long long)b * nz + k) * ny + j) * nx;
-      constexpr int xbytes = decltype(o.xt)::BYTES + (CMP ? decltype(o.lt)::BYTES : 0);
-      o.xt.setup(f3d_smem + warp * xbytes, lane_ok ? o.cp : nullptr, threadIdx.x & 31, nx);
       if constexpr (CMP) {
         o.lop = m.c32lo + (((long long)b * nz + k) * ny + j) * nx;
         o.r64 = m.rdxb64[0];
         o.r2 = m.rdxb2[0];
-        o.lt.setup(f3d_smem + warp * xbytes + decltype(o.xt)::BYTES, o.xt.rows,
-                   (long long)(m.c32lo - m.c32), threadIdx.x & 31, nx);
       }
       o.cs = 1;
       long long fo = (long long)k * (nx + 1) * ny + j;
@@ -380,7 +391,6 @@ __device__ __forceinline__ void sweep32_item(const MemberDev* __restrict__ membe
     } else if (DIR == DIR_Y) {
       i = (int)(pen % nx);
       int k = (int)(pen / nx);
-      n = ny;
       o.cp = m.c32 + ((long long)b * nz + k) * ny * (long long)nx + i;
       if constexpr (CMP) {
         o.lop = m.c32lo + ((long long)b * nz + k) * ny * (long long)nx + i;
@@ -396,7 +406,6 @@ __device__ __forceinline__ void sweep32_item(const MemberDev* __restrict__ membe
     } else {
       i = (int)(pen % nx);
       j = (int)(pen / nx);
-      n = nz;
       o.cp = m.c32 + (long long)b * nz * ny * nx + (long long)j * nx + i;
       if constexpr (CMP) {
         o.lop = m.c32lo + (long long)b * nz * ny * nx + (long long)j * nx + i;
@@ -410,6 +419,21 @@ __device__ __forceinline__ void sweep32_item(const MemberDev* __restrict__ membe
       o.vsub = m.vs32 + (long long)b * (nz + 1) * ny * nx + fo;
       area = m.dx2b[j + 1] * m.dx1b[i + 1];
       if constexpr (EPI) o.epi = zepi_setup(m, b, fo);
+    }
+    o.cp += (pstride_t)lo * o.cs;
+    o.fd += (pstride_t)lo * o.vs;
+    if (DIR == DIR_Z) o.vsub += (pstride_t)lo * o.vs;
+    if constexpr (CMP) {
+      o.lop += (pstride_t)lo * o.cs;
+      o.r64 += lo;
+      o.r2 += lo;
+    }
+    if constexpr (DIR == DIR_X) {
+      constexpr int xbytes = decltype(o.xt)::BYTES + (CMP ? decltype(o.lt)::BYTES : 0);
+      o.xt.setup(f3d_smem + warp * xbytes, lane_ok ? o.cp : nullptr, threadIdx.x & 31, n);
+      if constexpr (CMP)
+        o.lt.setup(f3d_smem + warp * xbytes + decltype(o.xt)::BYTES, o.xt.rows,
+                   (long long)(m.c32lo - m.c32), threadIdx.x & 31, n);
     }
     const double dt = m.dt;
     o.s1 = (float)m.stime;
@@ -476,14 +500,14 @@ template <int DIR, int LIM, int TM, bool CMP, bool EPI = false>
 __global__ void __launch_bounds__(128, CMP ? (DIR == DIR_X ? F3D_CMP_BLOCKS
                                                           : (DIR == DIR_Y ? F3D_CMP_Y_BLOCKS : F3D_CMP_YZ_BLOCKS))
                                               : 4)
-    k_sweep32(const MemberDev* __restrict__ members, const WorkItem* __restrict__ work, int bpb) {
+    k_sweep32(const MemberDev* __restrict__ members, const WorkItem* __restrict__ work, int bpb, const int2* __restrict__ ranges) {
   extern __shared__ __align__(16) unsigned char f3d_smem[];
-  sweep32_item<DIR, LIM, TM, CMP, EPI>(members, work[blockIdx.x], bpb, f3d_smem);
+  sweep32_item<DIR, LIM, TM, CMP, EPI>(members, work[blockIdx.x], bpb, ranges, f3d_smem);
 }
 
 template <int DIR, bool CMP, bool EPI = false>
 static void launch_dir32(int lim, int tm, const MemberDev* members, const WorkItem* work,
-                         int nblocks, int bpb, cudaStream_t st) {
+                         int nblocks, int bpb, const int2* ranges, cudaStream_t st) {
   dim3 g(nblocks), b(128);
   // RK4 x tiles keep one output buffer (XTile<float, 1>), Euler two; the
   // compensated form stages the low part as well, in chunks of F3D_CMP_XW
@@ -503,7 +527,7 @@ static void launch_dir32(int lim, int tm, const MemberDev* members, const WorkIt
     cudaFuncSetAttribute(k_sweep32<DIR, 3, 2, CMP>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_max);
     attr_set = true;
   }
-#define F3D_L(L, T) k_sweep32<DIR, L, T, CMP, EPI><<<g, b, smem, st>>>(members, work, bpb)
+#define F3D_L(L, T) k_sweep32<DIR, L, T, CMP, EPI><<<g, b, smem, st>>>(members, work, bpb, ranges)
   if (tm == 1) {
     if (lim == 1) F3D_L(1, 1); else if (lim == 2) F3D_L(2, 1); else F3D_L(3, 1);
   } else {
@@ -512,22 +536,33 @@ static void launch_dir32(int lim, int tm, const MemberDev* members, const WorkIt
 #undef F3D_L
 }
 
+// ranges: the work items' cells (launch_ranges32), null for all of them.
 // epi: the z sweep runs the wet deposition and decay epilogue (the members'
 // epi_on)
 void launch_sweep32(int dir, int lim, int tm, int cmp, int epi, const MemberDev* members,
-                    const WorkItem* work, int nblocks, int bpb, cudaStream_t st) {
+                    const WorkItem* work, int nblocks, int bpb, const int2* ranges, cudaStream_t st) {
   if (nblocks <= 0) return;
   if (cmp) {
-    if (dir == DIR_X) launch_dir32<DIR_X, true>(lim, tm, members, work, nblocks, bpb, st);
-    else if (dir == DIR_Y) launch_dir32<DIR_Y, true>(lim, tm, members, work, nblocks, bpb, st);
-    else if (epi) launch_dir32<DIR_Z, true, true>(lim, tm, members, work, nblocks, bpb, st);
-    else launch_dir32<DIR_Z, true>(lim, tm, members, work, nblocks, bpb, st);
+    if (dir == DIR_X) launch_dir32<DIR_X, true>(lim, tm, members, work, nblocks, bpb, ranges, st);
+    else if (dir == DIR_Y) launch_dir32<DIR_Y, true>(lim, tm, members, work, nblocks, bpb, ranges, st);
+    else if (epi) launch_dir32<DIR_Z, true, true>(lim, tm, members, work, nblocks, bpb, ranges, st);
+    else launch_dir32<DIR_Z, true>(lim, tm, members, work, nblocks, bpb, ranges, st);
   } else {
-    if (dir == DIR_X) launch_dir32<DIR_X, false>(lim, tm, members, work, nblocks, bpb, st);
-    else if (dir == DIR_Y) launch_dir32<DIR_Y, false>(lim, tm, members, work, nblocks, bpb, st);
-    else if (epi) launch_dir32<DIR_Z, false, true>(lim, tm, members, work, nblocks, bpb, st);
-    else launch_dir32<DIR_Z, false>(lim, tm, members, work, nblocks, bpb, st);
+    if (dir == DIR_X) launch_dir32<DIR_X, false>(lim, tm, members, work, nblocks, bpb, ranges, st);
+    else if (dir == DIR_Y) launch_dir32<DIR_Y, false>(lim, tm, members, work, nblocks, bpb, ranges, st);
+    else if (epi) launch_dir32<DIR_Z, false, true>(lim, tm, members, work, nblocks, bpb, ranges, st);
+    else launch_dir32<DIR_Z, false>(lim, tm, members, work, nblocks, bpb, ranges, st);
   }
+}
+
+// The boxes of every member's levels (maxlev: the most levels x bins of one),
+// and from them the ranges of the work items of the sweeps in dirs.
+void launch_ranges32(const MemberDev* members, int nmembers, int maxlev, const RangeArgs& a, cudaStream_t st) {
+  for (int f = 0; f < nmembers; f += 65535)
+    k_boxes32<<<dim3(maxlev, nmembers - f < 65535 ? nmembers - f : 65535), 256, 0, st>>>(members + f);
+  long long tot = 0;
+  for (int d = 0; d < 3; ++d) tot += (a.dirs >> d & 1) ? a.nwork[d] : 0;
+  k_ranges32<<<(int)((tot + 7) / 8), 256, 0, st>>>(members, a);
 }
 
 void launch_prep32(const MemberDev* members, const int* blk_member, const int* blk_first,
@@ -640,7 +675,7 @@ __device__ __forceinline__ void source32_all(MemberDev* members, int nmembers) {
 template <int DIR, int LIM, int TM, bool CMP, bool EPI = false>
 __device__ __noinline__ void sweep32_item_call(MemberDev* members, WorkItem w, int bpb,
                                                unsigned char* smem) {
-  sweep32_item<DIR, LIM, TM, CMP, EPI>(members, w, bpb, smem);
+  sweep32_item<DIR, LIM, TM, CMP, EPI>(members, w, bpb, nullptr, smem);
 }
 
 // One whole time step of every member in one persistent kernel: source,

@@ -216,6 +216,41 @@ void launch_face_kk(MemberDev* members, int mi, cudaStream_t st) {
   k_face_kk<<<1184, 256, 0, st>>>(members, mi);
 }
 
+// ---- MemberDev::wild: whether any face value or spacing is not below kCalm
+// (NaN and infinities included), once per change of the fields
+__global__ void k_field_bounds(const MemberDev* members, int mi, int* wild) {
+  const MemberDev& m = members[mi];
+  const long long nx = m.nx, ny = m.ny, nz = m.nz;
+  bool bad = false;
+  auto scan = [&](const double* p, long long n) {
+    GRID_STRIDE(e, n) bad = bad || !(fabs(p[e]) < kCalm);
+  };
+  auto spacing = [&](const double* p, long long n) {
+    GRID_STRIDE(e, n) bad = bad || !(fabs(p[e]) < kCalm && fabs(p[e]) > 1.0 / kCalm);
+  };
+  for (int s = 0; s < 2; ++s) {
+    scan(m.ux[s], (nx + 1) * ny * nz);
+    scan(m.vy[s], (ny + 1) * nx * nz);
+    scan(m.wz[s], (nz + 1) * nx * ny);
+  }
+  scan(m.k1x, (nx + 2) * ny * nz);
+  scan(m.k2y, (ny + 2) * nx * nz);
+  scan(m.k3z, (nz + 2) * nx * ny);
+  scan(m.vs, m.nb * (nz + 1) * nx * ny);
+  // dxp(p), p = -1..n-1, below the faces; dxb of the cells
+  spacing(m.dx1p + 1, nx + 1);
+  spacing(m.dx2p + 1, ny + 1);
+  spacing(m.dx3p + 1, nz + 1);
+  spacing(m.dx1b + 1, nx);
+  spacing(m.dx2b + 1, ny);
+  spacing(m.dx3b + 1, nz);
+  if (__any_sync(0xffffffffu, bad) && (threadIdx.x & 31) == 0) atomicExch(wild, 1);
+}
+void launch_field_bounds(MemberDev* members, int mi, int* wild, cudaStream_t st) {
+  cudaMemsetAsync(wild, 0, sizeof(int), st);
+  k_field_bounds<<<592, 256, 0, st>>>(members, mi, wild);
+}
+
 // ---- per-step parameters (kernel arguments are captured at launch) -------
 __global__ void k_set_step(MemberDev* members, int mi, double dt, double time, int iiter) {
   MemberDev& m = members[mi];

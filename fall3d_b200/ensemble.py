@@ -63,7 +63,8 @@ class Ensemble:
               "f3d_ens_create")
         self._h = h
         self.precision = precision
-        self.tuning = (MODE_KERNELS, 4, 0)  # the library's initial execution shape
+        # the library's initial execution shape (bins_per_block)
+        self.tuning = (MODE_KERNELS, 4 if nbins % 4 == 0 else 2 if nbins % 2 == 0 else 1, 0)
         self._keep = []
         for ci, g in enumerate(self.grids):
             arrs = [np.ascontiguousarray(getattr(g, n), dtype=np.float64) for n in

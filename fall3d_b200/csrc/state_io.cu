@@ -13,6 +13,8 @@
 
 #include <algorithm>
 #include <cstring>
+#include <memory>
+#include <new>
 #include <system_error>
 #include <thread>
 
@@ -112,11 +114,40 @@ static void place_rows(const RowsOut& r, const double* src, long long r0, long l
   }
 }
 
+// The same rows through ordinary memory, a megabyte at a time on the calling
+// thread: what is left where page-locked memory cannot be had.
+static cudaError_t download_pageable(const RowsOut& r, cudaStream_t st) {
+  const long long rows = r.ny * r.nz * r.nb;
+  const long long per = std::max<long long>(1, (1 << 17) / r.nx), most = std::min(rows, per) * r.nx;
+  std::unique_ptr<double[]> v(new (std::nothrow) double[most]);
+  std::unique_ptr<float[]> f(r.c64 ? nullptr : new (std::nothrow) float[2 * most]);
+  if (!v || (!r.c64 && !f)) return cudaErrorMemoryAllocation;
+  for (long long r0 = 0; r0 < rows; r0 += per) {
+    const long long r1 = std::min(rows, r0 + per), e0 = r0 * r.nx, cnt = (r1 - r0) * r.nx;
+    cudaError_t e;
+    if (r.c64) {
+      e = cudaMemcpyAsync(v.get(), r.c64 + e0, cnt * 8, cudaMemcpyDeviceToHost, st);
+    } else {
+      e = cudaMemcpyAsync(f.get(), r.c32 + e0, cnt * 4, cudaMemcpyDeviceToHost, st);
+      if (e == cudaSuccess && r.lo)
+        e = cudaMemcpyAsync(f.get() + most, r.lo + e0, cnt * 4, cudaMemcpyDeviceToHost, st);
+    }
+    if (e == cudaSuccess) e = cudaStreamSynchronize(st);
+    if (e != cudaSuccess) return e;
+    if (!r.c64)
+      for (long long q = 0; q < cnt; ++q) v[q] = r.lo ? (double)f[q] + (double)f[most + q] : (double)f[q];
+    place_rows(r, v.get(), r0, r1);
+  }
+  return cudaSuccess;
+}
+
 cudaError_t StateIO::download(const RowsOut& r, int device, cudaStream_t st) {
   const long long rows = r.ny * r.nz * r.nb;
   const size_t row = (size_t)r.nx * 8;
-  cudaError_t e = reserve(row * (size_t)rows, row);
-  if (e != cudaSuccess) return e;
+  if (reserve(row * (size_t)rows, row) != cudaSuccess) {
+    cudaGetLastError();
+    return download_pageable(r, st);
+  }
   const long long per = std::max<long long>(1, (long long)(slot_bytes_ / row));
   const long long chunks = (rows + per - 1) / per;
   // two slots a thread; a single thread below 8 MB, where starting others
@@ -151,12 +182,18 @@ cudaError_t StateIO::download(const RowsOut& r, int device, cudaStream_t st) {
 }
 
 cudaError_t StateIO::upload(void* dst, const void* src, size_t bytes, int device, cudaStream_t st) {
-  if (bytes < (4u << 20)) {  // the driver's own staging does as well here
-    cudaError_t e = cudaMemcpyAsync(dst, src, bytes, cudaMemcpyHostToDevice, st);
+  // small ones take the driver's own staging, which does as well there; so do
+  // all where page-locked memory cannot be had
+  bool slots = bytes >= (4u << 20);
+  if (slots && reserve(std::max(bytes, kSlots * kSlotBytes), 1) != cudaSuccess) {
+    cudaGetLastError();
+    slots = false;
+  }
+  cudaError_t e;
+  if (!slots) {
+    e = cudaMemcpyAsync(dst, src, bytes, cudaMemcpyHostToDevice, st);
     return e != cudaSuccess ? e : cudaStreamSynchronize(st);
   }
-  cudaError_t e = reserve(std::max(bytes, kSlots * kSlotBytes), 1);
-  if (e != cudaSuccess) return e;
   const long long per = (long long)slot_bytes_, chunks = ((long long)bytes + per - 1) / per;
   const int nth = (bytes < (8u << 20) || nslots_ < 4) ? 1 : nslots_ / 2;
   const int own = nth > 1 ? 2 : nslots_;

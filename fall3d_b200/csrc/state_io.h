@@ -43,7 +43,8 @@ class StateIO {
   ~StateIO() { release(); }
   // Both return cudaSuccess once the host array is complete (download) or the
   // host array may change again (upload; the device side is complete too).
-  // Work already on the stream comes first.
+  // Work already on the stream comes first.  Without page-locked memory both
+  // go through ordinary memory.
   cudaError_t download(const RowsOut& r, int device, cudaStream_t st);
   cudaError_t upload(void* dst, const void* src, size_t bytes, int device, cudaStream_t st);
   void release();

@@ -1,0 +1,98 @@
+"""State transfers where page-locked memory cannot be had: the library's own
+source, compiled for the host with an allocator that always fails and device
+memory played by host memory, must still move every value."""
+import subprocess
+
+import pytest
+
+from fall3d_b200 import build as B
+
+HARNESS = r"""
+#include <cuda_runtime.h>
+#include <cstdio>
+#include <cstring>
+#include <vector>
+static int pins = 0;
+static cudaError_t no_pin(void**, size_t) { ++pins; return cudaErrorMemoryAllocation; }
+static cudaError_t copy(void* d, const void* s, size_t n, cudaMemcpyKind, cudaStream_t) { memcpy(d, s, n); return cudaSuccess; }
+static cudaError_t fine() { return cudaSuccess; }
+#define cudaMallocHost no_pin
+#define cudaMemcpyAsync copy
+#define cudaStreamSynchronize(st) fine()
+#define cudaSetDevice(d) fine()
+#define cudaGetLastError() fine()
+#include "state_io.cu"
+using namespace f3d;
+
+// the interior and the two-deep face ghosts, everything else as it was
+static int wrong(const RowsOut& r, const std::vector<double>& host, const std::vector<double>& v) {
+  int bad = 0;
+  const bool halo = r.X != r.nx;
+  const long long h = halo ? 2 : 0, hz = r.Z != r.nz ? 2 : 0;
+  for (long long b = 0; b < r.nb; ++b)
+    for (long long k = 0; k < r.Z; ++k)
+      for (long long j = 0; j < r.Y; ++j)
+        for (long long i = 0; i < r.X; ++i) {
+          const long long q[3] = {i - h, j - h, k - hz}, n[3] = {r.nx, r.ny, r.nz};
+          long long at[3], out = 0;
+          for (int d = 0; d < 3; ++d) {
+            out += q[d] < 0 || q[d] >= n[d];
+            at[d] = q[d] < 0 ? 0 : q[d] >= n[d] ? n[d] - 1 : q[d];
+          }
+          const bool set = out == 0 || (out == 1 && r.faces);
+          const double want = set ? v[((b * r.nz + at[2]) * r.ny + at[1]) * r.nx + at[0]] : -7.0;
+          bad += host[((b * r.Z + k) * r.Y + j) * r.X + i] != want;
+        }
+  return bad;
+}
+
+int main() {
+  int bad = 0;
+  const long long shapes[][4] = {{5, 3, 2, 1}, {131, 70, 33, 5}, {200001, 2, 1, 1}};
+  for (auto& s : shapes)
+    for (int form = 0; form < 3; ++form) {
+      const long long nx = s[0], ny = s[1], nz = s[2], nb = s[3], n = nx * ny * nz * nb;
+      std::vector<double> c64(n), v(n);
+      std::vector<float> hi(n), lo(n);
+      for (long long q = 0; q < n; ++q) {
+        c64[q] = 1.0 / (q + 3);
+        hi[q] = (float)c64[q];
+        lo[q] = (float)(c64[q] - hi[q]);
+        v[q] = form == 0 ? c64[q] : form == 1 ? (double)hi[q] : (double)hi[q] + (double)lo[q];
+      }
+      MemberDev m{};
+      m.nx = (int)nx; m.ny = (int)ny; m.nz = (int)nz; m.nb = (int)nb;
+      if (form == 0) m.c64 = c64.data();
+      else m.c32 = hi.data();
+      if (form == 2) m.c32lo = lo.data();
+      std::vector<double> host((nx + 4) * (ny + 4) * (nz + 4) * nb, -7.0);
+      StateIO io;
+      const RowsOut r = rows3d(m, host.data(), true);
+      bad += io.download(r, 0, nullptr) != cudaSuccess;
+      bad += wrong(r, host, v);
+      if (form == 0) {
+        std::vector<double> a((nx + 4) * (ny + 4) * nb, -7.0), up(n, 0.0);
+        const RowsOut r2 = rows2d(c64.data(), nx, ny, nb, a.data());
+        bad += io.download(r2, 0, nullptr) != cudaSuccess;
+        std::vector<double> v2(v.begin(), v.begin() + nx * ny * nb);
+        bad += wrong(r2, a, v2);
+        bad += io.upload(up.data(), c64.data(), n * 8, 0, nullptr) != cudaSuccess;
+        bad += up != c64;
+      }
+    }
+  printf("pins %d bad %d\n", pins, bad);
+  return bad != 0 || pins == 0;
+}
+"""
+
+
+def test_without_page_locked_memory(tmp_path):
+    src, exe = tmp_path / "harness.cu", tmp_path / "harness"
+    src.write_text(HARNESS)
+    try:
+        nv = B.nvcc()
+    except RuntimeError:
+        pytest.skip("needs nvcc")
+    subprocess.run([nv, str(src), "-o", str(exe), "-O1", "-std=c++17", "-I" + B.CSRC] + B.ARCH, check=True)
+    r = subprocess.run([str(exe)], capture_output=True, text=True, timeout=60)
+    assert r.returncode == 0, r.stdout + r.stderr

@@ -13,9 +13,9 @@
 
 #include <algorithm>
 #include <cstring>
+#include <exception>
 #include <memory>
 #include <new>
-#include <system_error>
 #include <thread>
 
 namespace f3d {
@@ -77,7 +77,7 @@ static cudaError_t on_threads(int nthreads, W work) {
   for (int t = 1; t < nthreads; ++t) {
     try {
       th[t] = std::thread([&err, &work, t, nthreads] { err[t] = work(t, nthreads); });
-    } catch (const std::system_error&) {
+    } catch (const std::exception&) {  // no thread, or no memory for one
       here[t] = true;
     }
   }

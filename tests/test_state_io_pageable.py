@@ -1,6 +1,7 @@
-"""State transfers where page-locked memory cannot be had: the library's own
-source, compiled for the host with an allocator that always fails and device
-memory played by host memory, must still move every value."""
+"""State transfers where page-locked memory or threads cannot be had: the
+library's own source, compiled for the host with an allocator or threads that
+always fail and device memory played by host memory, must still move every
+value."""
 import subprocess
 
 import pytest
@@ -86,9 +87,58 @@ int main() {
 """
 
 
-def test_without_page_locked_memory(tmp_path):
+THREADS = r"""
+#include <cuda_runtime.h>
+#include <cstdlib>
+#include <cstring>
+#include <new>
+#include <thread>
+#include <vector>
+static cudaError_t pin(void** p, size_t n) { *p = malloc(n); return cudaSuccess; }
+static cudaError_t unpin(void* p) { free(p); return cudaSuccess; }
+static cudaError_t copy(void* d, const void* s, size_t n, cudaMemcpyKind, cudaStream_t) { memcpy(d, s, n); return cudaSuccess; }
+static cudaError_t event(cudaEvent_t* e, unsigned) { *e = (cudaEvent_t)1; return cudaSuccess; }
+static cudaError_t fine() { return cudaSuccess; }
+namespace std {
+struct no_thread {  // starts once, then finds no memory
+  static inline int made = 0;
+  std::thread t;
+  no_thread() = default;
+  template <class F>
+  explicit no_thread(F f) {
+    if (made++) throw std::bad_alloc();
+    t = std::thread(f);
+  }
+  void join() { t.join(); }
+};
+}
+#define cudaMallocHost pin
+#define cudaFreeHost unpin
+#define cudaMemcpyAsync copy
+#define cudaEventCreateWithFlags event
+#define cudaEventDestroy(e) fine()
+#define cudaEventRecord(e, st) fine()
+#define cudaEventSynchronize(e) fine()
+#define cudaStreamSynchronize(st) fine()
+#define cudaSetDevice(d) fine()
+#define thread no_thread
+#include "state_io.cu"
+
+int main() {
+  std::vector<char> a(20000003), b(a.size(), 0);
+  for (size_t q = 0; q < a.size(); ++q) a[q] = (char)(q * 2654435761u >> 13);
+  f3d::StateIO io;
+  const bool ok = io.upload(b.data(), a.data(), a.size(), 0, nullptr) == cudaSuccess && a == b;
+  return ok && std::no_thread::made == 3 ? 0 : 1;
+}
+"""
+
+
+# slots that cannot be page-locked; threads that cannot be started
+@pytest.mark.parametrize("harness", [HARNESS, THREADS], ids=["slots", "threads"])
+def test_transfers_without(tmp_path, harness):
     src, exe = tmp_path / "harness.cu", tmp_path / "harness"
-    src.write_text(HARNESS)
+    src.write_text(harness)
     try:
         nv = B.nvcc()
     except RuntimeError:

@@ -12,7 +12,9 @@
 // others march from eight cells before the box to eight after, and the zeros
 // around act as the ghost cells do (frozen values, no right-hand side).
 //
-// An eruption's plume fills a small part of its domain for most of a run.  On
+// The host asks for all this only where it pays (box_gate.h): a sweep without
+// ranges marches whole pencils.  An eruption's plume fills a small part of its
+// domain for most of a run.  On
 // the B200 the three compensated sweeps of a plume in 400 x 300 x 60 x 8 cells
 // went from 1.38 to 0.35 ms a step, with 0.08 ms for the boxes and ranges; with
 // ash everywhere (203 x 149 x 41 x 9) they went from 0.411 to 0.434 ms, with
@@ -151,21 +153,50 @@ __device__ __forceinline__ int2 box_range(const MemberDev& m, int dir, int b, in
 // spill 150-330 bytes and take up to 25% longer).  grown[d]: the directions
 // swept between the boxes and the sweep in d.  A warp per item.
 __global__ void __launch_bounds__(256) k_ranges32(const MemberDev* __restrict__ members, RangeArgs a) {
+  __shared__ unsigned int most[3], sum[3];
+  if (threadIdx.x < 3) most[threadIdx.x] = sum[threadIdx.x] = 0u;
+  __syncthreads();
   int q = blockIdx.x * 8 + (threadIdx.x >> 5), d = 0;
   for (; d < 3; ++d) {
     const int n = (a.dirs >> d & 1) ? a.nwork[d] : 0;
     if (q < n) break;
     q -= n;
   }
-  if (d == 3) return;
-  const WorkItem w = a.work[d][q];
-  int lo = 0x7fffffff, hi = 0;
-  for (int s = 0; s < 4; ++s) {
-    const int2 r = box_range(members[w.member], d, w.bin0 + s % a.bpb, w.pen0 + 32 * (s / a.bpb), a.grown[d]);
-    lo = min(lo, r.x);
-    hi = max(hi, r.y);
+  if (d < 3) {
+    const WorkItem w = a.work[d][q];
+    int lo = 0x7fffffff, hi = 0;
+    for (int s = 0; s < 4; ++s) {
+      const int2 r = box_range(members[w.member], d, w.bin0 + s % a.bpb, w.pen0 + 32 * (s / a.bpb), a.grown[d]);
+      lo = min(lo, r.x);
+      hi = max(hi, r.y);
+    }
+    if ((threadIdx.x & 31) == 0) {
+      a.range[d][q] = lo < hi ? make_int2(lo, hi) : make_int2(0, 0);
+      if (lo < hi) {
+        atomicMax(&most[d], (unsigned int)(hi - lo));
+        atomicAdd(&sum[d], (unsigned int)(hi - lo));
+      }
+    }
   }
-  if ((threadIdx.x & 31) == 0) a.range[d][q] = lo < hi ? make_int2(lo, hi) : make_int2(0, 0);
+  __syncthreads();
+  // the lengths of all items for the host (box_gate.h), by the last block
+  if (threadIdx.x != 0) return;
+  for (int e = 0; e < 3; ++e)
+    if (sum[e]) {
+      atomicMax(a.acc + e, most[e]);
+      atomicAdd(a.acc + 3 + e, sum[e]);
+    }
+  __threadfence();
+  if (atomicAdd(a.acc + 6, 1u) != gridDim.x - 1) return;
+  __threadfence();
+  volatile unsigned int* pub = a.pub;
+  for (int e = 0; e < 6; ++e) pub[1 + e] = atomicExch(a.acc + e, 0u);
+  pub[7] = (unsigned int)a.dirs;
+  a.acc[6] = 0u;
+  const unsigned int run = a.acc[7] + 1u;
+  a.acc[7] = run;
+  __threadfence_system();
+  pub[0] = run;
 }
 
 }  // namespace f3d

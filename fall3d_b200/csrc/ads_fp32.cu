@@ -337,9 +337,10 @@ __device__ __forceinline__ void block_reduce2_f64(double a, double b, double* ou
 
 // One work item (32 pencils x bpb bins of one member) of a sweep; called by
 // the per-sweep kernels and by the persistent fused step kernel.  EPI (z
-// only): the wet deposition and decay epilogue, a kernel instance of its own
-// so that the sweeps without it keep their register allocation.
-template <int DIR, int LIM, int TM, bool CMP = false, bool EPI = false>
+// only): the wet deposition and decay epilogue; RANGED: the march over the
+// item's range of cells alone.  Both are kernel instances of their own, so
+// that the sweeps without them keep their register allocation.
+template <int DIR, int LIM, int TM, bool CMP = false, bool EPI = false, bool RANGED = false>
 __device__ __forceinline__ void sweep32_item(const MemberDev* __restrict__ members,
                                              const WorkItem w, int bpb,
                                              const int2* __restrict__ ranges, unsigned char* f3d_smem) {
@@ -356,10 +357,10 @@ __device__ __forceinline__ void sweep32_item(const MemberDev* __restrict__ membe
   const long long pen = pen_raw < nsp ? pen_raw : nsp - 1;
   double clo = 0.0, chi = 0.0;
   // the cells this sweep can change: positions 0..n-1 of the march are
-  // act.x..act.y-1 of the pencil (the epilogue counts levels: all of them)
+  // act.x..act.y-1 of the pencil
   int2 act = make_int2(0, (DIR == DIR_X) ? nx : (DIR == DIR_Y) ? ny : nz);
-  if (!EPI && ranges) act = __ldg(ranges + blockIdx.x);
-  if (act.x == act.y) {
+  if constexpr (RANGED) act = __ldg(ranges + blockIdx.x);
+  if (RANGED && act.x == act.y) {
     if (lane_ok && m.gh32) {  // an empty pencil's ghosts
       float* g = m.gh32 + (long long)b * gh_per_bin(nx, ny, nz);
       g[gh_offset(DIR, 0, pen, nx, ny, nz)] = 0.f;
@@ -371,19 +372,23 @@ __device__ __forceinline__ void sweep32_item(const MemberDev* __restrict__ membe
   if (run_it) {
     Ops32<LIM, DIR, TM, CMP, EPI> o;
     double area;
-    const int lo = act.x, n = act.y - act.x;
+    const int lo = RANGED ? act.x : 0, n = RANGED ? act.y - act.x : (DIR == DIR_X) ? nx : (DIR == DIR_Y) ? ny : nz;
     int i = 0, j = 0;
     if (DIR == DIR_X) {
       j = (int)(pen % ny);
       int k = (int)(pen / ny);
-      o.cp = m.c32 + (((long long)b * nz + k) * ny + j) * nx;
+      o.cp = m.c32 + (((long long)b * nz + k) * ny + j) * nx + lo;
+      constexpr int xbytes = decltype(o.xt)::BYTES + (CMP ? decltype(o.lt)::BYTES : 0);
+      o.xt.setup(f3d_smem + warp * xbytes, lane_ok ? o.cp : nullptr, threadIdx.x & 31, n);
       if constexpr (CMP) {
-        o.lop = m.c32lo + (((long long)b * nz + k) * ny + j) * nx;
-        o.r64 = m.rdxb64[0];
-        o.r2 = m.rdxb2[0];
+        o.lop = m.c32lo + (((long long)b * nz + k) * ny + j) * nx + lo;
+        o.r64 = m.rdxb64[0] + lo;
+        o.r2 = m.rdxb2[0] + lo;
+        o.lt.setup(f3d_smem + warp * xbytes + decltype(o.xt)::BYTES, o.xt.rows,
+                   (long long)(m.c32lo - m.c32), threadIdx.x & 31, n);
       }
       o.cs = 1;
-      long long fo = (long long)k * (nx + 1) * ny + j;
+      long long fo = (long long)k * (nx + 1) * ny + j + (long long)lo * ny;
       o.fd = (m.gc_cur ? m.gc4[0] : m.f4[0]) + fo;
       o.vs = ny;
       o.vsub = nullptr;
@@ -420,20 +425,15 @@ __device__ __forceinline__ void sweep32_item(const MemberDev* __restrict__ membe
       area = m.dx2b[j + 1] * m.dx1b[i + 1];
       if constexpr (EPI) o.epi = zepi_setup(m, b, fo);
     }
-    o.cp += (pstride_t)lo * o.cs;
-    o.fd += (pstride_t)lo * o.vs;
-    if (DIR == DIR_Z) o.vsub += (pstride_t)lo * o.vs;
-    if constexpr (CMP) {
-      o.lop += (pstride_t)lo * o.cs;
-      o.r64 += lo;
-      o.r2 += lo;
-    }
-    if constexpr (DIR == DIR_X) {
-      constexpr int xbytes = decltype(o.xt)::BYTES + (CMP ? decltype(o.lt)::BYTES : 0);
-      o.xt.setup(f3d_smem + warp * xbytes, lane_ok ? o.cp : nullptr, threadIdx.x & 31, n);
-      if constexpr (CMP)
-        o.lt.setup(f3d_smem + warp * xbytes + decltype(o.xt)::BYTES, o.xt.rows,
-                   (long long)(m.c32lo - m.c32), threadIdx.x & 31, n);
+    if constexpr (RANGED && DIR != DIR_X) {  // x: above, where its staging starts from the row
+      o.cp += (pstride_t)lo * o.cs;
+      o.fd += (pstride_t)lo * o.vs;
+      if (DIR == DIR_Z) o.vsub += (pstride_t)lo * o.vs;
+      if constexpr (CMP) {
+        o.lop += (pstride_t)lo * o.cs;
+        o.r64 += lo;
+        o.r2 += lo;
+      }
     }
     const double dt = m.dt;
     o.s1 = (float)m.stime;
@@ -492,7 +492,7 @@ __device__ __forceinline__ void sweep32_item(const MemberDev* __restrict__ membe
 #ifndef F3D_CMP_YZ_BLOCKS
 #define F3D_CMP_YZ_BLOCKS 4
 #endif
-template <int DIR, int LIM, int TM, bool CMP, bool EPI = false>
+template <int DIR, int LIM, int TM, bool CMP, bool EPI = false, bool RANGED = false>
 // 4 blocks of 128 threads per SM (128 registers); with one output buffer the
 // RK4 x tiles (4 x 12.6 KB per block) fit 4 blocks as well.  The compensated
 // x sweep runs 4 blocks too: at 128 registers it spills a few bytes, and it
@@ -500,13 +500,14 @@ template <int DIR, int LIM, int TM, bool CMP, bool EPI = false>
 __global__ void __launch_bounds__(128, CMP ? (DIR == DIR_X ? F3D_CMP_BLOCKS
                                                           : (DIR == DIR_Y ? F3D_CMP_Y_BLOCKS : F3D_CMP_YZ_BLOCKS))
                                               : 4)
-    k_sweep32(const MemberDev* __restrict__ members, const WorkItem* __restrict__ work, int bpb, const int2* __restrict__ ranges) {
+    k_sweep32(const MemberDev* __restrict__ members, const WorkItem* __restrict__ work, int bpb,
+              const int2* __restrict__ ranges) {
   extern __shared__ __align__(16) unsigned char f3d_smem[];
-  sweep32_item<DIR, LIM, TM, CMP, EPI>(members, work[blockIdx.x], bpb, ranges, f3d_smem);
+  sweep32_item<DIR, LIM, TM, CMP, EPI, RANGED>(members, work[blockIdx.x], bpb, ranges, f3d_smem);
 }
 
-template <int DIR, bool CMP, bool EPI = false>
-static void launch_dir32(int lim, int tm, const MemberDev* members, const WorkItem* work,
+template <int DIR, bool CMP, bool EPI, bool RANGED>
+static void launch_form32(int lim, int tm, const MemberDev* members, const WorkItem* work,
                          int nblocks, int bpb, const int2* ranges, cudaStream_t st) {
   dim3 g(nblocks), b(128);
   // RK4 x tiles keep one output buffer (XTile<float, 1>), Euler two; the
@@ -519,15 +520,15 @@ static void launch_dir32(int lim, int tm, const MemberDev* members, const WorkIt
                        : 0;
   static bool attr_set = false;
   if (!attr_set && smem_max > 0) {
-    cudaFuncSetAttribute(k_sweep32<DIR, 1, 1, CMP>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_max);
-    cudaFuncSetAttribute(k_sweep32<DIR, 2, 1, CMP>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_max);
-    cudaFuncSetAttribute(k_sweep32<DIR, 3, 1, CMP>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_max);
-    cudaFuncSetAttribute(k_sweep32<DIR, 1, 2, CMP>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_max);
-    cudaFuncSetAttribute(k_sweep32<DIR, 2, 2, CMP>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_max);
-    cudaFuncSetAttribute(k_sweep32<DIR, 3, 2, CMP>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_max);
+    cudaFuncSetAttribute(k_sweep32<DIR, 1, 1, CMP, EPI, RANGED>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_max);
+    cudaFuncSetAttribute(k_sweep32<DIR, 2, 1, CMP, EPI, RANGED>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_max);
+    cudaFuncSetAttribute(k_sweep32<DIR, 3, 1, CMP, EPI, RANGED>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_max);
+    cudaFuncSetAttribute(k_sweep32<DIR, 1, 2, CMP, EPI, RANGED>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_max);
+    cudaFuncSetAttribute(k_sweep32<DIR, 2, 2, CMP, EPI, RANGED>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_max);
+    cudaFuncSetAttribute(k_sweep32<DIR, 3, 2, CMP, EPI, RANGED>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_max);
     attr_set = true;
   }
-#define F3D_L(L, T) k_sweep32<DIR, L, T, CMP, EPI><<<g, b, smem, st>>>(members, work, bpb, ranges)
+#define F3D_L(L, T) k_sweep32<DIR, L, T, CMP, EPI, RANGED><<<g, b, smem, st>>>(members, work, bpb, ranges)
   if (tm == 1) {
     if (lim == 1) F3D_L(1, 1); else if (lim == 2) F3D_L(2, 1); else F3D_L(3, 1);
   } else {
@@ -536,21 +537,28 @@ static void launch_dir32(int lim, int tm, const MemberDev* members, const WorkIt
 #undef F3D_L
 }
 
+template <int DIR, bool CMP>
+static void launch_dir32(int lim, int tm, const MemberDev* members, const WorkItem* work,
+                         int nblocks, int bpb, const int2* ranges, cudaStream_t st) {
+  if (ranges) launch_form32<DIR, CMP, false, true>(lim, tm, members, work, nblocks, bpb, ranges, st);
+  else launch_form32<DIR, CMP, false, false>(lim, tm, members, work, nblocks, bpb, nullptr, st);
+}
+
 // ranges: the work items' cells (launch_ranges32), null for all of them.
 // epi: the z sweep runs the wet deposition and decay epilogue (the members'
-// epi_on)
+// epi_on) and, as that counts levels, all cells
 void launch_sweep32(int dir, int lim, int tm, int cmp, int epi, const MemberDev* members,
                     const WorkItem* work, int nblocks, int bpb, const int2* ranges, cudaStream_t st) {
   if (nblocks <= 0) return;
   if (cmp) {
     if (dir == DIR_X) launch_dir32<DIR_X, true>(lim, tm, members, work, nblocks, bpb, ranges, st);
     else if (dir == DIR_Y) launch_dir32<DIR_Y, true>(lim, tm, members, work, nblocks, bpb, ranges, st);
-    else if (epi) launch_dir32<DIR_Z, true, true>(lim, tm, members, work, nblocks, bpb, ranges, st);
+    else if (epi) launch_form32<DIR_Z, true, true, false>(lim, tm, members, work, nblocks, bpb, nullptr, st);
     else launch_dir32<DIR_Z, true>(lim, tm, members, work, nblocks, bpb, ranges, st);
   } else {
     if (dir == DIR_X) launch_dir32<DIR_X, false>(lim, tm, members, work, nblocks, bpb, ranges, st);
     else if (dir == DIR_Y) launch_dir32<DIR_Y, false>(lim, tm, members, work, nblocks, bpb, ranges, st);
-    else if (epi) launch_dir32<DIR_Z, false, true>(lim, tm, members, work, nblocks, bpb, ranges, st);
+    else if (epi) launch_form32<DIR_Z, false, true, false>(lim, tm, members, work, nblocks, bpb, nullptr, st);
     else launch_dir32<DIR_Z, false>(lim, tm, members, work, nblocks, bpb, ranges, st);
   }
 }

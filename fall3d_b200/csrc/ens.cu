@@ -17,6 +17,7 @@
 #include <vector>
 
 #include "../../include/fall3d_ads.h"
+#include "box_gate.h"
 #include "f3d_common.cuh"
 #include "phys_dev.cuh"
 #include "phys_host.h"
@@ -153,6 +154,11 @@ struct f3d_ens {
   WorkItem* dwork[3] = {nullptr, nullptr, nullptr};
   int2* drange[3] = {nullptr, nullptr, nullptr};  // precision form: the work items' cells
   int nwork[3] = {0, 0, 0};
+  BoxGate gate;                    // whether a step looks for its boxes
+  unsigned int* d_gate = nullptr;
+  unsigned int* h_gate = nullptr;  // page-locked, in h_pin
+  int march_longest[3] = {0, 0, 0};
+  long long march_total[3] = {0, 0, 0};  // cells all blocks march in whole pencils
   int* dprep_member = nullptr;
   int* dprep_first = nullptr;
   int nprep = 0;
@@ -173,8 +179,9 @@ struct f3d_ens {
   StateIO io;  // transfers of the members' host arrays
   int iiter = 0;
   bool dm_valid = false;  // the device member table has been written once
-  cudaGraphExec_t graph[2] = {nullptr, nullptr};
-  bool graph_ok = false;
+  // step graphs: x or y first (persistent mode: [0] for both), without and
+  // with the boxes; a pair is captured when a step first needs one of it
+  cudaGraphExec_t graph[2][2] = {{nullptr, nullptr}, {nullptr, nullptr}};
   int fused_grid = 0;
   long long launches = 0;
   std::vector<void*> work_allocs;  // rebuilt with the tuning
@@ -214,12 +221,12 @@ int ealloc(f3d_ens* e, T** p, size_t n) {
 }
 
 void drop_graphs(f3d_ens* e) {
-  for (auto& g : e->graph)
-    if (g) {
-      cudaGraphExecDestroy(g);
-      g = nullptr;
-    }
-  e->graph_ok = false;
+  for (auto& boxes : e->graph)
+    for (auto& g : boxes)
+      if (g) {
+        cudaGraphExecDestroy(g);
+        g = nullptr;
+      }
 }
 
 int update_radio_factors(f3d_ens* e, const double* dt);
@@ -254,6 +261,7 @@ int upload_members(f3d_ens* e) {
 // fields at the same place run back to back.  Flux slots stay contiguous
 // per member.
 int build_work(f3d_ens* e) {
+  e->gate.reset();
   for (void* p : e->work_allocs) cudaFree(p);
   e->work_allocs.clear();
   const int bpb = e->bpb;
@@ -262,11 +270,16 @@ int build_work(f3d_ens* e) {
   int slot = 0;
   std::vector<std::vector<WorkItem>> lists(3);
   for (int d = 0; d < 3; ++d) {
+    e->march_longest[d] = 0;
+    e->march_total[d] = 0;
     for (int mi = 0; mi < e->nm; ++mi) {
       const EnsClass& c = e->cls[e->member_class[mi]];
       long long nsp = d == 0 ? (long long)c.ny * c.nz : d == 1 ? (long long)c.nx * c.nz
                                                                : (long long)c.nx * c.ny;
       const int ng = (int)((nsp + span - 1) / span);
+      const int n = d == 0 ? c.nx : d == 1 ? c.ny : c.nz;
+      e->march_longest[d] = std::max(e->march_longest[d], n);
+      e->march_total[d] += (long long)ng * nbg * n;
       e->hm[mi].part_base[d] = slot;
       e->hm[mi].part_count[d] = ng * nbg;
       slot += ng * nbg;
@@ -445,6 +458,7 @@ extern "C" int f3d_ens_create(int nclasses, const f3d_dims* dims, int nmembers,
   rc |= ealloc(e, &e->d_err, 1);
   rc |= ealloc(e, &e->d_nfail, 4);
   rc |= ealloc(e, &e->d_wild, (size_t)nclasses);
+  if (f32) rc |= ealloc(e, &e->d_gate, kGateWords);
   rc |= ealloc(e, &e->staging, stage + 4 * (size_t)nb);
   e->staging_elems = stage;
   for (int m = 0; m < nmembers && !rc; ++m) {
@@ -506,7 +520,13 @@ extern "C" int f3d_ens_create(int nclasses, const f3d_dims* dims, int nmembers,
     rc |= cudaMemsetAsync(e->d_err, 0, 4, e->st) != cudaSuccess;
     rc |= cudaMemsetAsync(e->d_wild, 0xff, 4 * (size_t)nclasses, e->st) != cudaSuccess;  // until set
     e->h_pin_elems = 16 * (size_t)nmembers + 64;
-    rc |= cudaMallocHost(&e->h_pin, e->h_pin_elems * 8) != cudaSuccess;
+    rc |= cudaMallocHost(&e->h_pin, e->h_pin_elems * 8 + 4 * kGateWords) != cudaSuccess;
+  }
+  if (!rc && e->d_gate) {
+    e->h_gate = reinterpret_cast<unsigned int*>(e->h_pin + e->h_pin_elems);
+    std::fill(e->h_gate, e->h_gate + kGateWords, 0u);
+    rc |= cudaMemsetAsync(e->d_gate, 0, 4 * kGateWords, e->st) != cudaSuccess;
+    e->gate.attach(e->h_gate, cmp);
   }
   if (!rc) rc |= ealloc(e, &e->dm, (size_t)nmembers);
   if (!rc) rc |= build_work(e);
@@ -899,6 +919,7 @@ extern "C" int f3d_ens_upload_member_state(f3d_ens* e, int mi, const double* my_
       ECK(cudaMemcpy(m.c32, tmp.data(), tmp.size() * 4, cudaMemcpyHostToDevice));
       if (m.c32lo) ECK(cudaMemcpy(m.c32lo, tlo.data(), tlo.size() * 4, cudaMemcpyHostToDevice));
     }
+    e->gate.reset();
   }
   if (my_acum && ens_upload_conv(e, k, 8, my_acum, (nx + 4) * (ny + 4) * nb, m.acum)) return 1;
   if (my_c && (m.gh64 || m.gh32)) {  // the halo cells of the given state
@@ -1177,7 +1198,12 @@ int wet_radio_launches(const f3d_ens* e) {
   return n;
 }
 
-int enqueue_step(f3d_ens* e, bool xfirst, bool advance, cudaEvent_t* ev = nullptr,
+// Whether the next step's sweeps march over the boxes (precision form, per-phase kernels).
+bool step_boxes(f3d_ens* e) {
+  return e->prec == F3D_PREC_FP32 && e->gate.use(7, e->march_longest, e->march_total);
+}
+
+int enqueue_step(f3d_ens* e, bool xfirst, bool boxes, bool advance, cudaEvent_t* ev = nullptr,
                  const std::vector<std::pair<int, GcArgs>>* gcl = nullptr) {
   if (ev) ECK(cudaEventRecord(ev[0], e->st));
   // a step with the gravity current runs the per-phase kernels, which take
@@ -1218,8 +1244,8 @@ int enqueue_step(f3d_ens* e, bool xfirst, bool advance, cudaEvent_t* ev = nullpt
     }
   }
   if (e->prec == F3D_PREC_FP64) launch_source64(e->dm, e->nm, e->st);
-  else {
-    launch_source32(e->dm, e->nm, e->st);
+  else launch_source32(e->dm, e->nm, e->st);
+  if (boxes) {
     RangeArgs a;
     for (int d = 0; d < 3; ++d) {
       a.work[d] = e->dwork[d];
@@ -1231,9 +1257,11 @@ int enqueue_step(f3d_ens* e, bool xfirst, bool advance, cudaEvent_t* ev = nullpt
     a.grown[DIR_X] = xfirst ? 0 : 1 << DIR_Y;
     a.grown[DIR_Y] = xfirst ? 1 << DIR_X : 0;
     a.grown[DIR_Z] = 1 << DIR_X | 1 << DIR_Y;
+    a.acc = e->d_gate;
+    a.pub = e->h_gate;
     launch_ranges32(e->dm, e->nm, e->maxlev, a, e->st);
   }
-  e->launches += (e->prec == F3D_PREC_FP64) ? 2 : 3;
+  e->launches += (e->prec == F3D_PREC_FP64) ? 2 : boxes ? 3 : 1;
   if (ev) ECK(cudaEventRecord(ev[1], e->st));
   const int order[3] = {xfirst ? DIR_X : DIR_Y, xfirst ? DIR_Y : DIR_X, DIR_Z};
   for (int q = 0; q < 3; ++q) {
@@ -1242,7 +1270,7 @@ int enqueue_step(f3d_ens* e, bool xfirst, bool advance, cudaEvent_t* ev = nullpt
       launch_sweep64(d, e->lim, e->tm, e->hm[0].epi_on, e->dm, e->dwork[d], e->nwork[d], e->bpb, e->st);
     else
       launch_sweep32(d, e->lim, e->tm, e->cmp, e->hm[0].epi_on, e->dm, e->dwork[d], e->nwork[d], e->bpb,
-                     e->drange[d], e->st);
+                     boxes ? e->drange[d] : nullptr, e->st);
     e->launches += 1;
     if (ev) ECK(cudaEventRecord(ev[2 + q], e->st));
   }
@@ -1280,33 +1308,32 @@ int accumulate_profile(f3d_ens* e, bool xfirst) {
   return 0;
 }
 
-int build_graphs(f3d_ens* e) {
-  drop_graphs(e);
-  const int ng = (e->mode == F3D_ENS_MODE_PERSISTENT) ? 1 : 2;
-  for (int q = 0; q < ng; ++q) {
-    cudaGraph_t g = nullptr;
-    ECK(cudaStreamBeginCapture(e->st, cudaStreamCaptureModeThreadLocal));
-    long long keep = e->launches;
-    int rc = enqueue_step(e, q == 0, true);
-    cudaError_t ce = cudaStreamEndCapture(e->st, &g);
-    e->launches = keep;
-    if (rc || ce != cudaSuccess) {
-      if (g) cudaGraphDestroy(g);
-      cudaGetLastError();
-      return set_error_msg("step graph capture failed: %s", cudaGetErrorString(ce));
-    }
-    cudaError_t ie = cudaGraphInstantiate(&e->graph[q], g, 0);
-    cudaGraphDestroy(g);
-    if (ie != cudaSuccess) return set_error_msg("graph instantiation failed: %s", cudaGetErrorString(ie));
+// Capture of one step graph: e->graph[boxes][order].
+int build_graph(f3d_ens* e, bool boxes, int order) {
+  if (e->graph[boxes][order]) return 0;
+  cudaGraph_t g = nullptr;
+  ECK(cudaStreamBeginCapture(e->st, cudaStreamCaptureModeThreadLocal));
+  long long keep = e->launches;
+  int rc = enqueue_step(e, order == 0, boxes, true);
+  cudaError_t ce = cudaStreamEndCapture(e->st, &g);
+  e->launches = keep;
+  if (rc || ce != cudaSuccess) {
+    if (g) cudaGraphDestroy(g);
+    cudaGetLastError();
+    return set_error_msg("step graph capture failed: %s", cudaGetErrorString(ce));
   }
-  if (ng == 1) e->graph[1] = nullptr;
-  e->graph_ok = true;
+  cudaError_t ie = cudaGraphInstantiate(&e->graph[boxes][order], g, 0);
+  cudaGraphDestroy(g);
+  if (ie != cudaSuccess) {
+    e->graph[boxes][order] = nullptr;
+    return set_error_msg("graph instantiation failed: %s", cudaGetErrorString(ie));
+  }
   return 0;
 }
 
-int kernels_per_step(const f3d_ens* e) {
+int kernels_per_step(const f3d_ens* e, bool boxes) {
   if (e->mode == F3D_ENS_MODE_PERSISTENT) return 1 + wet_radio_launches(e);
-  return (e->prec == F3D_PREC_FP64 ? 2 : 3) + 3 + 1 + 1 + wet_radio_launches(e);
+  return (e->prec == F3D_PREC_FP64 ? 2 : boxes ? 3 : 1) + 3 + 1 + 1 + wet_radio_launches(e);
 }
 
 }  // namespace
@@ -1323,17 +1350,20 @@ extern "C" int f3d_ens_run(f3d_ens* e, int nsteps) {
   if (e->prof) {
     for (int s = 0; s < nsteps; ++s) {
       const bool xfirst = (e->mode == F3D_ENS_MODE_PERSISTENT) || (e->iiter % 2 == 0);
-      if (enqueue_step(e, xfirst, true, e->pev)) return 1;
+      if (enqueue_step(e, xfirst, step_boxes(e), true, e->pev)) return 1;
       if (accumulate_profile(e, xfirst)) return 1;
       e->iiter += 1;
     }
     return 0;
   }
-  if (!e->graph_ok && build_graphs(e)) return 1;
   for (int s = 0; s < nsteps; ++s) {
-    cudaGraphExec_t g = (e->mode == F3D_ENS_MODE_PERSISTENT) ? e->graph[0] : e->graph[e->iiter & 1];
-    ECK(cudaGraphLaunch(g, e->st));
-    e->launches += kernels_per_step(e);
+    const bool persistent = e->mode == F3D_ENS_MODE_PERSISTENT, boxes = !persistent && step_boxes(e);
+    const int order = persistent ? 0 : e->iiter & 1;
+    if (!e->graph[boxes][order])  // both orders, so that no step after this one waits for a capture
+      for (int q = 0; q < (persistent ? 1 : 2); ++q)
+        if (build_graph(e, boxes, q)) return 1;
+    ECK(cudaGraphLaunch(e->graph[boxes][order], e->st));
+    e->launches += kernels_per_step(e, boxes);
     e->iiter += 1;
   }
   return 0;
@@ -1554,11 +1584,13 @@ extern "C" int f3d_ens_autotune(f3d_ens* e, int steps, const char* cache_file, c
     const int* c = kTuneCand[q];
     int derr = 0;
     float el = 0.f;
-    // warm-up step (builds the graphs), then `steps` timed steps on the
-    // ensemble's stream; a candidate that fails or whose barriers gave up
-    // is skipped
+    // a warm-up step that tells whether the boxes pay and one as the later
+    // steps run (they build the graphs), then `steps` timed steps on the
+    // ensemble's stream; a candidate that fails or whose barriers gave up is
+    // skipped
     if (f3d_ens_set_tuning(e, c[0], c[1], c[2]) || f3d_ens_run(e, 1) ||
-        cudaEventRecord(ev[0], e->st) != cudaSuccess || f3d_ens_run(e, steps) ||
+        cudaStreamSynchronize(e->st) != cudaSuccess || f3d_ens_run(e, 1) ||
+        cudaStreamSynchronize(e->st) != cudaSuccess || cudaEventRecord(ev[0], e->st) != cudaSuccess || f3d_ens_run(e, steps) ||
         cudaEventRecord(ev[1], e->st) != cudaSuccess || f3d_ens_status(e, &derr) ||
         cudaEventElapsedTime(&el, ev[0], ev[1]) != cudaSuccess) {
       cudaGetLastError();
@@ -1607,7 +1639,7 @@ extern "C" int f3d_ens_step(f3d_ens* e, const double* dt, const double* time, in
   launch_set_steps(e->dm, e->nm, dt, time, iiter, e->st);
   e->launches += (e->nm + 63) / 64;
   ECKL();
-  if (enqueue_step(e, iiter % 2 == 0, false, nullptr, &gcl)) return 1;
+  if (enqueue_step(e, iiter % 2 == 0, step_boxes(e), false, nullptr, &gcl)) return 1;
   e->iiter = iiter + 1;
   if (fluxes) {
     ECK(cudaMemcpyAsync(e->h_pin, e->flux_step, 6 * (size_t)e->nm * 8, cudaMemcpyDeviceToHost, e->st));
@@ -1670,6 +1702,7 @@ extern "C" int f3d_ens_reset_state(f3d_ens* e) {
   ECK(cudaMemsetAsync(e->flux_tot, 0, 12 * (size_t)e->nm * 8, e->st));
   ECK(cudaMemsetAsync(e->flux_step, 0, 6 * (size_t)e->nm * 8, e->st));
   ECK(cudaStreamSynchronize(e->st));
+  e->gate.reset();
   return 0;
 }
 

@@ -13,6 +13,7 @@
 #include <vector>
 
 #include "../../include/fall3d_ads.h"
+#include "box_gate.h"
 #include "f3d_common.cuh"
 #include "phys_dev.cuh"
 #include "phys_host.h"
@@ -139,6 +140,10 @@ struct f3d_ctx {
   WorkItem* dwork[3] = {nullptr, nullptr, nullptr};
   int2* drange[3] = {nullptr, nullptr, nullptr};  // precision form: the work items' cells
   int nblk[3] = {0, 0, 0};
+  BoxGate gate;                  // whether a step looks for its boxes
+  unsigned int* d_gate = nullptr;
+  unsigned int* h_gate = nullptr;  // page-locked
+  long long march_total[3] = {0, 0, 0};  // cells all blocks march in whole pencils
   int* dprep_member = nullptr;
   int* dprep_first = nullptr;
   int nprep = 0;
@@ -234,6 +239,7 @@ static int build_work(f3d_ctx* c) {
     if (c->prec == F3D_PREC_FP32 && dalloc(c, &c->drange[d], (size_t)nb)) return 1;
     CK(cudaMemcpy(c->dwork[d], w.data(), sizeof(WorkItem) * nb, cudaMemcpyHostToDevice));
     c->nblk[d] = nb;
+    c->march_total[d] = (long long)nb * (d == 0 ? c->nx : d == 1 ? c->ny : c->nz);
   }
   if (dalloc(c, &c->hm.flux_part, 2 * (size_t)slot)) return 1;
   long long nprep = ((long long)(c->nx + 1) * c->ny * c->nz + (long long)(c->ny + 1) * c->nx * c->nz +
@@ -379,6 +385,7 @@ extern "C" int f3d_ads_create(const f3d_dims* dims, int limiter, int time_marchi
   rc |= dalloc(c, &c->d_red, (size_t)c->mass_nblk * nb + 64);
   rc |= dalloc(c, &c->d_nfail, 4);
   rc |= dalloc(c, &c->d_wild, 1);
+  if (precision == F3D_PREC_FP32) rc |= dalloc(c, &c->d_gate, kGateWords);
   if (precision == F3D_PREC_FP32) m.wild = c->d_wild;
   size_t stage = std::max({(nx + 4) * (ny + 4) * (nz + 4) * nb, nx * ny * (nz + 3) * nb,
                            2 * (nx + 3) * ny * nz, 2 * (ny + 3) * nx * nz, 2 * (nz + 3) * nx * ny,
@@ -387,7 +394,8 @@ extern "C" int f3d_ads_create(const f3d_dims* dims, int limiter, int time_marchi
   c->staging_elems = stage;
   rc |= dalloc(c, &c->dm, 1);
   if (rc == 0) rc |= build_work(c);
-  if (rc == 0 && cudaMallocHost(&c->h_pin, 4096) != cudaSuccess) rc = set_err("pinned alloc failed");
+  if (rc == 0 && cudaMallocHost(&c->h_pin, 4096 + 4 * kGateWords) != cudaSuccess)
+    rc = set_err("pinned alloc failed");
   if (rc) {
     std::string keep = g_err;
     f3d_ads_destroy(c);
@@ -399,6 +407,12 @@ extern "C" int f3d_ads_create(const f3d_dims* dims, int limiter, int time_marchi
   if (m.c32lo) CK(cudaMemsetAsync(m.c32lo, 0, ncell * nb * sizeof(float), c->st));
   CK(cudaMemsetAsync(m.acum, 0, nx * ny * nb * sizeof(double), c->st));
   CK(cudaMemsetAsync(c->d_wild, 0xff, sizeof(int), c->st));  // until the fields are set
+  if (c->d_gate) {
+    c->h_gate = reinterpret_cast<unsigned int*>(c->h_pin + 512);
+    std::fill(c->h_gate, c->h_gate + kGateWords, 0u);
+    CK(cudaMemsetAsync(c->d_gate, 0, sizeof(unsigned int) * kGateWords, c->st));
+    c->gate.attach(c->h_gate, c->cmp != 0);
+  }
   CK(cudaMemsetAsync(m.flux_tot, 0, 12 * sizeof(double), c->st));
   CK(cudaMemsetAsync(m.flux_step, 0, 6 * sizeof(double), c->st));
   if (upload_member(c)) return 1;
@@ -1137,6 +1151,7 @@ extern "C" int f3d_ads_upload_state(f3d_ctx* c, const double* my_c, const double
       CK(cudaMemcpy(m.c32, tmp.data(), tmp.size() * 4, cudaMemcpyHostToDevice));
       if (m.c32lo) CK(cudaMemcpy(m.c32lo, tlo.data(), tlo.size() * 4, cudaMemcpyHostToDevice));
     }
+    c->gate.reset();
   }
   if (my_acum && upload_conv(c, 8, my_acum, (nx + 4) * (ny + 4) * nb, m.acum)) return 1;
   if (my_c && (m.gh64 || m.gh32)) {
@@ -1174,9 +1189,12 @@ extern "C" int f3d_ads_download_state(f3d_ctx* c, double* my_c, double* my_acum)
 }
 
 // ---- step ---------------------------------------------------------------
-// The ranges of the sweeps in dirs (precision form), x before y or after it.
-static int enqueue_ranges(f3d_ctx* c, int dirs, bool xfirst) {
-  if (c->prec != F3D_PREC_FP32) return 0;
+// The ranges of the sweeps in dirs, x before y or after it, where they are
+// taken to pay (precision form, BoxGate); *on says whether they were.
+static int enqueue_ranges(f3d_ctx* c, int dirs, bool xfirst, bool* on) {
+  const int longest[3] = {c->nx, c->ny, c->nz};
+  *on = c->prec == F3D_PREC_FP32 && c->gate.use(dirs, longest, c->march_total);
+  if (!*on) return 0;
   RangeArgs a;
   for (int d = 0; d < 3; ++d) {
     a.work[d] = c->dwork[d];
@@ -1188,19 +1206,21 @@ static int enqueue_ranges(f3d_ctx* c, int dirs, bool xfirst) {
   a.grown[DIR_X] = dirs & (xfirst ? 0 : 1 << DIR_Y);
   a.grown[DIR_Y] = dirs & (xfirst ? 1 << DIR_X : 0);
   a.grown[DIR_Z] = dirs & (1 << DIR_X | 1 << DIR_Y);
+  a.acc = c->d_gate;
+  a.pub = c->h_gate;
   launch_ranges32(c->dm, 1, c->nb * c->nz, a, c->st);
   c->launches += 2;
   CKL();
   return 0;
 }
 
-static int enqueue_sweep(f3d_ctx* c, int dir) {
+static int enqueue_sweep(f3d_ctx* c, int dir, bool boxes) {
   c->launches += 1;
   if (c->prec == F3D_PREC_FP64)
     launch_sweep64(dir, c->lim, c->tm, c->hm.epi_on, c->dm, c->dwork[dir], c->nblk[dir], c->bpb, c->st);
   else
     launch_sweep32(dir, c->lim, c->tm, c->cmp, c->hm.epi_on, c->dm, c->dwork[dir], c->nblk[dir], c->bpb,
-                   c->drange[dir], c->st);
+                   boxes ? c->drange[dir] : nullptr, c->st);
   CKL();
   return 0;
 }
@@ -1366,13 +1386,14 @@ static int enqueue_step(f3d_ctx* c, double dt, double time, int iiter) {
   }
   if (enqueue_source(c)) return 1;
   const bool xfirst = (iiter % 2 == 0);  // mod_F3D.F90:1477-1487
-  if (enqueue_ranges(c, 7, xfirst)) return 1;
+  bool boxes;
+  if (enqueue_ranges(c, 7, xfirst, &boxes)) return 1;
   rec(1);
-  if (enqueue_sweep(c, xfirst ? DIR_X : DIR_Y)) return 1;
+  if (enqueue_sweep(c, xfirst ? DIR_X : DIR_Y, boxes)) return 1;
   rec(2);
-  if (enqueue_sweep(c, xfirst ? DIR_Y : DIR_X)) return 1;
+  if (enqueue_sweep(c, xfirst ? DIR_Y : DIR_X, boxes)) return 1;
   rec(3);
-  if (enqueue_sweep(c, DIR_Z)) return 1;
+  if (enqueue_sweep(c, DIR_Z, boxes)) return 1;
   rec(4);
   launch_flux_reduce(c->dm, 1, 7, c->st);
   c->launches += 1;
@@ -1473,7 +1494,8 @@ static int solve_dir(f3d_ctx* c, int dir, double dt, double* a, double* b, const
   if (check_ready(c, who)) return 1;
   if (!a || !b) return set_err("%s: null flux argument", who);
   CK(cudaSetDevice(c->device));
-  if (enqueue_ranges(c, 1 << dir, true) || enqueue_sweep(c, dir)) return 1;
+  bool boxes;
+  if (enqueue_ranges(c, 1 << dir, true, &boxes) || enqueue_sweep(c, dir, boxes)) return 1;
   launch_flux_reduce(c->dm, 1, 1 << dir, c->st);
   CKL();
   CK(cudaMemcpyAsync(c->h_pin, c->hm.flux_step, 6 * sizeof(double), cudaMemcpyDeviceToHost, c->st));

@@ -260,6 +260,8 @@ struct RangeArgs {
   int2* range[3];
   int nwork[3], grown[3];
   int dirs, bpb;
+  unsigned int* acc;  // [kGateWords] in device memory, zero between runs but for the last (box_gate.h)
+  unsigned int* pub;  // [kGateWords] page-locked: what the host reads
 };
 
 // Host: bins per sweep block (its four warps take that many bins of one tile

@@ -586,7 +586,7 @@ int f3d_ens_gravity_current_time_steps(f3d_ens *ens, const double *times, const 
 /* Autotuner of the batched step (no counterpart in the reference, whose
  * members run as separate jobs).  Times each candidate execution shape on
  * the device -- per-phase kernels replayed from CUDA graphs with 4, 2 or 1
- * bins per block, the persistent step kernel with 4 or 2 -- for one warm-up
+ * bins per block, the persistent step kernel with 4 or 2 -- for two warm-up
  * and `steps` timed steps (CUDA events on the ensemble's stream), keeps the
  * fastest and sets it.  Member state and clocks advance while tuning: reset
  * them afterwards if needed.  With cache_file and key (a single token, e.g.

@@ -587,12 +587,15 @@ int f3d_ens_gravity_current_time_steps(f3d_ens *ens, const double *times, const 
  * members run as separate jobs).  Times each candidate execution shape on
  * the device -- per-phase kernels replayed from CUDA graphs with 4, 2 or 1
  * bins per block, the persistent step kernel with 4 or 2 -- for two warm-up
- * and `steps` timed steps (CUDA events on the ensemble's stream), keeps the
- * fastest and sets it.  Member state and clocks advance while tuning: reset
- * them afterwards if needed.  With cache_file and key (a single token, e.g.
- * class shapes, bins, precision and GPU name) the result is read from and
- * written to that text file, so a later run with the same key sets the
- * cached shape without timing.  tuning[3] = {mode, bins per block, blocks
+ * and `steps` timed steps (CUDA events on the ensemble's stream), all of them
+ * there and back (first to last, last to first), keeps the fastest mean and
+ * sets it.  Member state and clocks advance while tuning: reset them
+ * afterwards if needed.  In the precision forms the per-phase kernels skip
+ * cells without ash and the persistent kernel does not, so the times, also
+ * those in the cache, are those of the state that was there.  With cache_file
+ * and key (a single token, e.g. class shapes, bins, precision and GPU name)
+ * the result is read from and written to that text file, so a later run with
+ * the same key sets the cached shape without timing.  tuning[3] = {mode, bins per block, blocks
  * per SM (0 = as many as fit)}; cand_ms (may be NULL) receives the
  * F3D_ENS_TUNE_CANDIDATES candidates' ms per step (-1 where one failed). */
 #define F3D_ENS_TUNE_CANDIDATES 5

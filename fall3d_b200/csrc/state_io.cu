@@ -6,9 +6,11 @@
 // host array is made on the way (a fresh 460 MB vector costs more in page
 // faults than its whole transfer), and large transfers are copied by four
 // threads with two slots each: one slot fills while the other is emptied.
-// On the B200 the 503 MB state of a 400 x 300 x 60 x 8 domain arrives in ~25 ms
-// (one thread through several host vectors: ~465 ms), the winds, densities and
-// settling velocities of a 200 x 150 x 40 x 8 meteo update in ~15 ms (~55 ms).
+// On the B200 a state of 400 x 300 x 60 x 4 cells (230 MB) arrives in 16 ms,
+// in 10.6 through the larger slots (130 through host vectors in one thread); a
+// context's first read-back of 60 x 45 x 40 x 8 (7 MB) in 0.9 ms (1.7 through
+// vectors, 9.2 with the larger slots from the start); the corner fields of a
+// 200 x 150 x 40 meteo update go up in 7.6 ms (36 stacked and pageable).
 #include "state_io.h"
 
 #include <algorithm>
@@ -36,14 +38,20 @@ __global__ void k_rows_out(const double* __restrict__ c64, const float* __restri
 }
 
 cudaError_t StateIO::reserve(size_t total, size_t unit) {
-  size_t slot = std::max(unit, std::min(kSlotBytes, total));
+  moved_ += std::min(total, kLargeFrom);  // no overflow in the longest run
+  moved_ = std::min(moved_, kLargeFrom);
+  const bool large = !no_large_ && moved_ >= kLargeFrom && total >= kSlots * kLargeSlotBytes;
+  const size_t slot = std::max(unit, std::min(large ? kLargeSlotBytes : kSlotBytes, total));
   const int n = (int)std::min<size_t>(kSlots, (total + slot - 1) / slot);
   if (slot <= slot_bytes_ && n <= nslots_) return cudaSuccess;
   release();
   cudaError_t e = cudaMallocHost((void**)&pin_, slot * n);
   if (e != cudaSuccess) {
     pin_ = nullptr;
-    return e;
+    if (!large) return e;
+    cudaGetLastError();
+    no_large_ = true;
+    return reserve(total, unit);
   }
   for (int s = 0; s < n; ++s)
     if ((e = cudaEventCreateWithFlags(&ev_[s], cudaEventDisableTiming)) != cudaSuccess) {
@@ -185,7 +193,7 @@ cudaError_t StateIO::upload(void* dst, const void* src, size_t bytes, int device
   // small ones take the driver's own staging, which does as well there; so do
   // all where page-locked memory cannot be had
   bool slots = bytes >= (4u << 20);
-  if (slots && reserve(std::max(bytes, kSlots * kSlotBytes), 1) != cudaSuccess) {
+  if (slots && reserve(bytes, 1) != cudaSuccess) {
     cudaGetLastError();
     slots = false;
   }

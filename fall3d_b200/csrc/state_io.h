@@ -50,12 +50,20 @@ class StateIO {
   void release();
 
  private:
-  static constexpr int kSlots = 8;             // two per host thread
-  static constexpr size_t kSlotBytes = 1 << 20;  // page-locking costs ~0.5 ms a MB, once
+  static constexpr int kSlots = 8;  // two per host thread
+  // Eight slots of 192 KB come with the 2 MB that the driver page-locks for
+  // the context's first small allocation, so that the first transfer of a
+  // context takes no longer than the later ones.  Slots of 1 MB cost 5-10 ms
+  // to page-lock and save 2.5 ms per 100 MB, so they are taken once a context
+  // has moved 384 MB.
+  static constexpr size_t kSlotBytes = 192 << 10, kLargeSlotBytes = 1 << 20;
+  static constexpr size_t kLargeFrom = 384 << 20;
   cudaError_t reserve(size_t total, size_t unit);
   char* pin_ = nullptr;
   size_t slot_bytes_ = 0;
   int nslots_ = 0;
+  size_t moved_ = 0;  // bytes that went through reserve(), up to kLargeFrom
+  bool no_large_ = false;  // the large slots could not be had
   cudaEvent_t ev_[kSlots] = {};
 };
 

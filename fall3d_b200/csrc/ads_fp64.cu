@@ -66,6 +66,7 @@ struct Ops64 {
   pstride64_t vs;
   const double* kk;    // 0.5 (k(f) + k(f-1)) at face f, same stride
   const double4* geo;  // {dxp(p), 1/dxp(p), dxb(p), 1/dxb(p)} at geo[p + 1]
+  unsigned int small;  // high word of the numerators that take rhs_small
   int nf;              // cells of the pencil (faces 0..nf)
   double dt, hdt;
   XTile<double> xt;    // x pencils: shared-memory staging of the rows
@@ -143,9 +144,17 @@ struct Ops64 {
       const double F_r = cr * u;
       const double F0 = 0.5 * (F_l + F_r) - 0.5 * fabs(u) * (cr - cl);
       const double4 g = geo[min(max(p + 1, 0), nf)];
-      const double P0 = div_rn_geo(fv.k * s.d1, g.x, g.y);
+      const double n = fv.k * s.d1, dF = F0 - s.F1;
+      double P0 = div_rn_geo(n, g.x, g.y);
+      const double dP = P0 - s.P1;
+      double d = div_rn_geo(dP, g.z, g.w) - div_rn_geo(dF, g.z, g.w);
+      if (below_nonzero(n, small) || below_nonzero(dP, small) || below_nonzero(dF, small)) {
+        const double2 t = rhs_small(n, s.P1, dF, g.x, g.y, g.z, g.w);
+        P0 = t.x;
+        d = t.y;
+      }
       flux = F0 + P0;
-      if (!G || q >= 2) rhs = div_rn_geo(P0 - s.P1, g.z, g.w) - div_rn_geo(F0 - s.F1, g.z, g.w);
+      if (!G || q >= 2) rhs = d;
       if (!G) rhs = (p >= 0 && p < nf) ? rhs : 0.0;  // ghost cells of the unguarded march
       s.F1 = F0;
       s.P1 = P0;
@@ -228,6 +237,7 @@ __device__ __forceinline__ void sweep64_pencil(const MemberDev& m, long long pen
     if constexpr (EPI) o.epi = zepi_setup(m, b, fo);
   }
   o.geo = m.geo[DIR];
+  o.small = (unsigned int)__double2hiint(o.geo[n + 1].x);
   o.nf = n;
   o.dt = m.dt;
   o.hdt = 0.5 * m.dt;

@@ -421,9 +421,9 @@ extern "C" int f3d_ens_create(int nclasses, const f3d_dims* dims, int nmembers,
       rc |= ealloc(e, &k.kkf[0], fu);
       rc |= ealloc(e, &k.kkf[1], fv);
       rc |= ealloc(e, &k.kkf[2], fw);
-      rc |= ealloc(e, &k.geo[0], nx + 1);
-      rc |= ealloc(e, &k.geo[1], ny + 1);
-      rc |= ealloc(e, &k.geo[2], nz + 1);
+      rc |= ealloc(e, &k.geo[0], nx + 2);
+      rc |= ealloc(e, &k.geo[1], ny + 2);
+      rc |= ealloc(e, &k.geo[2], nz + 2);
     } else {
       rc |= ealloc(e, &k.f4[0], fu);
       rc |= ealloc(e, &k.f4[1], fv);
@@ -566,14 +566,17 @@ extern "C" int f3d_ens_set_class_grid(f3d_ens* e, int ci, const double* dX1_p, c
   const size_t nn[3] = {nx, ny, nz};
   for (int d = 0; d < 3; ++d) {
     if (e->prec == F3D_PREC_FP64) {
-      std::vector<double4> g(nn[d] + 1);
+      std::vector<double4> g(nn[d] + 2);
+      double most = 0.0;
       for (size_t q = 0; q <= nn[d]; ++q) {
         double a = dp[d][q + 1], b = db[d][q];
         if (!(std::fabs(a) >= 0x1p-100 && std::fabs(a) <= 0x1p100 && std::fabs(b) >= 0x1p-100 &&
               std::fabs(b) <= 0x1p100))
           return set_error_msg("f3d_ens_set_class_grid: spacing outside [2^-100, 2^100]");
         g[q] = make_double4(a, 1.0 / a, b, 1.0 / b);
+        most = std::max(most, std::max(std::fabs(a), std::fabs(b)));
       }
+      g[nn[d] + 1] = make_double4(div_small(most), 0.0, 0.0, 0.0);
       ECK(cudaMemcpy(k.geo[d], g.data(), g.size() * sizeof(double4), cudaMemcpyHostToDevice));
     } else {
       std::vector<float> r(nn[d]);

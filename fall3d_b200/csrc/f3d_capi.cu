@@ -347,9 +347,9 @@ extern "C" int f3d_ads_create(const f3d_dims* dims, int limiter, int time_marchi
     rc |= dalloc(c, &tmp, (ny + 1) * nx * nz); m.kkf[1] = tmp;
     rc |= dalloc(c, &tmp, (nz + 1) * nx * ny); m.kkf[2] = tmp;
     double4* g4;
-    rc |= dalloc(c, &g4, nx + 1); m.geo[0] = g4;
-    rc |= dalloc(c, &g4, ny + 1); m.geo[1] = g4;
-    rc |= dalloc(c, &g4, nz + 1); m.geo[2] = g4;
+    rc |= dalloc(c, &g4, nx + 2); m.geo[0] = g4;
+    rc |= dalloc(c, &g4, ny + 2); m.geo[1] = g4;
+    rc |= dalloc(c, &g4, nz + 2); m.geo[2] = g4;
   } else {
     float* f;
     float4* f4;
@@ -464,19 +464,23 @@ extern "C" int f3d_ads_set_grid(f3d_ctx* c, const double* dX1_p, const double* d
   c->Hm3_p.assign(Hm3_p, Hm3_p + nx * ny);
   if (c->prec == F3D_PREC_FP64) {
     // geo[p+1] = {dxp(p), RN(1/dxp(p)), dxb(p), RN(1/dxb(p))}, p = -1..n-1
-    // (reference offsets +2 / +1); the reciprocals feed div_rn_recip
+    // (reference offsets +2 / +1), for the divisions of ads_fp64.cu, and their
+    // div_small()
     const double* dp[3] = {dX1_p, dX2_p, dX3_p};
     const double* db[3] = {dX1_b, dX2_b, dX3_b};
     const size_t nn[3] = {nx, ny, nz};
     for (int d = 0; d < 3; ++d) {
-      std::vector<double4> g(nn[d] + 1);
+      std::vector<double4> g(nn[d] + 2);
+      double most = 0.0;
       for (size_t q = 0; q <= nn[d]; ++q) {
         double a = dp[d][q + 1], b = db[d][q];
         if (!(std::fabs(a) >= 0x1p-100 && std::fabs(a) <= 0x1p100 && std::fabs(b) >= 0x1p-100 &&
               std::fabs(b) <= 0x1p100))
           return set_err("f3d_ads_set_grid: grid spacing %g / %g outside [2^-100, 2^100]", a, b);
         g[q] = make_double4(a, 1.0 / a, b, 1.0 / b);
+        most = std::max(most, std::max(std::fabs(a), std::fabs(b)));
       }
+      g[nn[d] + 1] = make_double4(div_small(most), 0.0, 0.0, 0.0);
       CK(cudaMemcpy((void*)m.geo[d], g.data(), g.size() * sizeof(double4), cudaMemcpyHostToDevice));
     }
   }

@@ -52,7 +52,8 @@ struct MemberDev {
   const double* k3z;
   const double* vs;
   // FP64 face data of the exact form, per direction (0 x, 1 y, 2 z):
-  //   geo[d][p+1] = {dxp(p), 1/dxp(p), dxb(p), 1/dxb(p)} for p = -1..n-1
+  //   geo[d][p+1] = {dxp(p), 1/dxp(p), dxb(p), 1/dxb(p)} for p = -1..n-1,
+  //   geo[d][n+1].x = div_small() of them
   //   kkf[d] = 0.5 (k(f) + k(f-1)) at every face, laid out like the winds
   const double4* geo[3];
   const double* kkf[3];
@@ -306,31 +307,66 @@ __device__ __forceinline__ double div_rn_recip(double a, double b, double y) {
   return (a == 0.0) ? a * y : res;
 }
 
-// Non-zero and below 2^(E - 1023).  On the integer pipe.
-template <unsigned int E>
-__device__ __forceinline__ bool below_nonzero(double a) {
-  const unsigned int hi = (unsigned int)__double2hiint(a) & 0x7fffffffu;
-  return hi < (E << 20) && (hi | (unsigned int)__double2loint(a)) != 0u;
+// Non-zero and below the power of two whose high word is `hi`.  On the integer pipe.
+__device__ __forceinline__ bool below_nonzero(double a, unsigned int hi) {
+  const unsigned int m = (unsigned int)__double2hiint(a) & 0x7fffffffu;
+  return m < hi && (m | (unsigned int)__double2loint(a)) != 0u;
 }
-static __device__ __noinline__ double div_rn_tiny(double a, double b, double y) { return div_rn_recip(a, b, y); }
 
-// The same quotient with the rare numerators out of the way: q = a y and
+// a/b as in div_rn_recip for |a| < 2^500, scaled whatever its size: no select,
+// and a branch for the tie alone (one for every subnormal result makes the
+// sweeps of a wide plume 10% slower: they are frequent and diverge).
+__device__ __forceinline__ double div_rn_scaled(double a, double b, double y) {
+  const double sa = a * 0x1p400;
+  double q = sa * y;
+  double r = fma(-q, b, sa);
+  q = fma(r, y, q);
+  r = fma(-q, b, sa);
+  q = fma(r, y, q);
+  double res = q * 0x1p-400;
+  const double d = fma(-res, 0x1p400, q);  // exact; 0 where the result is normal
+  if (fabs(d) == 0x1p-675) {
+    const double rem = fma(-q, b, sa);  // exact
+    if (rem != 0.0 && ((d > 0.0) == ((rem > 0.0) == (b > 0.0)))) res = res + copysign(0x1p-1074, d);
+  }
+  return res;
+}
+
+// The quotient with the rare numerators out of the way: q = a y and
 // Markstein's two corrections, five operations where the selects, scalings
-// and the tie of div_rn_recip make it ten to sixteen.  From 2^-900 on nothing
-// leaves the normal range (|b| in [2^-100, 2^100]: q >= 2^-1000, and the
-// remainder is a multiple of 2^-104 |a| / 4).  A zero numerator gives a zero
-// of either sign, which no sum of the sweeps tells apart.  With div_rn_3 and
-// div_rn_6 below: the y sweep of 157 x 93 x 37 x 5 cells full of ash 310 ->
-// 232 us, z 411 -> 338, x 624 -> 528; a plume's far fringe, where many values
-// take the long way, gains less.
+// and the tie of div_rn_recip make it ten to sixteen.  Correctly rounded while
+// nothing leaves the normal range: |a| not below div_small(...) of the
+// spacings, or zero.  A zero numerator gives a zero of either sign, which no
+// sum of the sweeps tells apart.
 __device__ __forceinline__ double div_rn_geo(double a, double b, double y) {
   double q = a * y;
   double r = fma(-q, b, a);
   q = fma(r, y, q);
   r = fma(-q, b, a);
-  q = fma(r, y, q);
-  if (below_nonzero<1023 - 900>(a)) q = div_rn_tiny(a, b, y);
-  return q;
+  return fma(r, y, q);
+}
+// Host: the numerators div_rn_geo can take for spacings of at most `most`.
+// The quotient is normal from 2^-1022 on, and the remainder, a multiple of
+// ulp(q) ulp(b) >= 2^-106 |a|, is representable while that is 2^-1074 or more:
+// |a| >= 2^-966 for |b| <= 2^50, 2^-920 for |b| <= 2^100 (the largest taken).
+inline double div_small(double most) { return most <= 0x1p50 ? 0x1p-966 : 0x1p-920; }
+
+// A cell's diffusive flux P0 = n / dxp and right-hand side (P0 - P1) / dxb -
+// dF / dxb where one of the three numerators is small: one call for the three
+// divisions.  With a call for each the steps of wide plumes, whose fringe is
+// full of such values, took up to a fifth longer than with div_rn_recip
+// everywhere (y of 301 x 227 x 37 x 4: 1.15 to 1.51 ms; 1.23 with the one
+// call, later scaled and less often needed); inline in each place it costs 255
+// registers and 7 minutes of compiling for no gain.
+static __device__ __noinline__ double2 rhs_small(double n, double P1, double dF, double dxp, double rdxp, double dxb,
+                                                 double rdxb) {
+  // the scaled quotients stay below 2^1001
+  if (fabs(n) < 0x1p400 && fabs(P1) < 0x1p499 && fabs(dF) < 0x1p500) {
+    const double P0 = div_rn_scaled(n, dxp, rdxp);
+    return make_double2(P0, div_rn_scaled(P0 - P1, dxb, rdxb) - div_rn_scaled(dF, dxb, rdxb));
+  }
+  const double P0 = div_rn_recip(n, dxp, rdxp);
+  return make_double2(P0, div_rn_recip(P0 - P1, dxb, rdxb) - div_rn_recip(dF, dxb, rdxb));
 }
 
 // Correctly rounded a / 3 and a / 6 in two operations: a z + (a z') with z + z'
@@ -338,19 +374,22 @@ __device__ __forceinline__ double div_rn_geo(double a, double b, double y) {
 // correctly rounded floating-point division when the divisor is known in
 // advance", IEEE Trans. Computers 53(8), 2004).  z = RN(1/3) has 3 z = 1 -
 // 2^-54, so 1/3 - z = 2^-54 / 3 and z' = RN of that = 2^-54 z.  Before its
-// rounding the sum is off by less than 2^-105 |a|; a / 3 is a multiple of 1/3
-// of half an ulp of the quotient and no midpoint itself, so it is 1/6 ulp or
-// more away from every midpoint, and the rounding falls on its side.  Dividing
-// by 2 is exact.
+// rounding the sum is off by less than 2^-105 |a|, and by 2^-1075 more where a
+// z' is subnormal; a / 3 is a multiple of 1/3 of half an ulp of the quotient
+// and no midpoint itself, so it is 1/6 ulp or more away from every midpoint,
+// and the rounding falls on its side while an ulp of the quotient is 2^-1072
+// or more: |a| >= 2^-1010 is.  Dividing by 2 is exact.
+constexpr unsigned int kSmall36 = (1023u - 1010u) << 20;
+static __device__ __noinline__ double div_rn_small(double a, double b, double y) { return div_rn_scaled(a, b, y); }
 __device__ __forceinline__ double div_rn_3(double a) {
   constexpr double z = 0x1.5555555555555p-2;
   const double q = fma(a, z, a * (z * 0x1p-54));
-  return below_nonzero<1023 - 960>(a) ? div_rn_tiny(a, 3.0, 1.0 / 3.0) : q;
+  return below_nonzero(a, kSmall36) ? div_rn_small(a, 3.0, 1.0 / 3.0) : q;
 }
 __device__ __forceinline__ double div_rn_6(double a) {
   constexpr double z = 0x1.5555555555555p-3;
   const double q = fma(a, z, a * (z * 0x1p-54));
-  return below_nonzero<1023 - 960>(a) ? div_rn_tiny(a, 6.0, 1.0 / 6.0) : q;
+  return below_nonzero(a, kSmall36) ? div_rn_small(a, 6.0, 1.0 / 6.0) : q;
 }
 
 }  // namespace f3d

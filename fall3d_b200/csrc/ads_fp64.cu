@@ -296,12 +296,16 @@ __global__ void __launch_bounds__(128, MINB) k_sweep64(const MemberDev* __restri
   sweep64_item<DIR, LIM, TM, EPI>(members, work[blockIdx.x], bpb, f3d_smem);
 }
 
-// Blocks per SM of an RK4 sweep.  The march waits more than it computes, so a
-// round of resident blocks takes about as long per block held: 0.49 ms with
-// two on an SM, 0.72 with three (x of 200 x 150 x 40 x 8).  What counts is how
-// the blocks divide into rounds: 375 of them are two rounds of 296 or one of
-// 444 (0.97 against 0.71 ms), 135 are one round either way (x of 157 x 93 x
-// 37 x 5: 0.53 against 0.69 ms).  With many rounds the two come out alike.
+// Blocks per SM of an RK4 sweep: what counts is how the blocks divide into
+// rounds of resident ones.  The march waits more than it computes, so a round
+// with three on an SM takes 1.07 to 1.35 times one with two (y of 100 x 80 x 40
+// x 6: 151 and 133 us; x of 157 x 93 x 37 x 5: 457 and 366).  Three where they
+// make fewer rounds than two by 1.3: z of 157 x 93 x 37 x 8, 3 rounds against 4,
+// 377 against 402 us; y of 200 x 150 x 40 x 12 and of 400 x 300 x 60 x 4, 2
+// against 3, 649 against 791 and 1186 against 1489; z of 200 x 150 x 40 x 12, 7
+// against 10, 830 against 948; z of 400 x 300 x 60 x 4, 9 against 13, 1692
+// against 1754.  Two where the rounds are as many (x of 200 x 150 x 40 x 12: 2,
+// 873 against 1118).
 static int blocks_per_sm(int nblocks) {
   static const int nsm = [] {
     int dev = 0, n = 0;
@@ -311,7 +315,7 @@ static int blocks_per_sm(int nblocks) {
     return n;
   }();
   const int two = (nblocks + 2 * nsm - 1) / (2 * nsm), three = (nblocks + 3 * nsm - 1) / (3 * nsm);
-  return 3 * three < 2 * two ? 3 : 2;
+  return 13LL * three < 10LL * two ? 3 : 2;
 }
 
 // Host launchers -------------------------------------------------------------

@@ -189,23 +189,27 @@ cudaError_t StateIO::download(const RowsOut& r, int device, cudaStream_t st) {
   });
 }
 
+static bool page_locked(const void* p) {
+  cudaPointerAttributes a;
+  if (cudaPointerGetAttributes(&a, p) == cudaSuccess) return a.type == cudaMemoryTypeHost;
+  cudaGetLastError();
+  return false;
+}
+
 cudaError_t StateIO::upload(void* dst, const void* src, size_t bytes, int device, cudaStream_t st) {
   // small ones take the driver's own staging, which does as well there; so do
-  // all where page-locked memory cannot be had
-  bool slots = bytes >= (4u << 20);
+  // all where page-locked memory cannot be had, and a caller's page-locked
+  // array needs none
+  bool slots = bytes >= (4u << 20) && !page_locked(src);
   if (slots && reserve(bytes, 1) != cudaSuccess) {
     cudaGetLastError();
     slots = false;
   }
-  cudaError_t e;
-  if (!slots) {
-    e = cudaMemcpyAsync(dst, src, bytes, cudaMemcpyHostToDevice, st);
-    return e != cudaSuccess ? e : cudaStreamSynchronize(st);
-  }
+  if (!slots) return cudaMemcpyAsync(dst, src, bytes, cudaMemcpyHostToDevice, st);
   const long long per = (long long)slot_bytes_, chunks = ((long long)bytes + per - 1) / per;
   const int nth = (bytes < (8u << 20) || nslots_ < 4) ? 1 : nslots_ / 2;
   const int own = nth > 1 ? 2 : nslots_;
-  e = on_threads(nth, [&](int t, int n) -> cudaError_t {
+  const cudaError_t e = on_threads(nth, [&](int t, int n) -> cudaError_t {
     cudaError_t err = cudaSetDevice(device);
     if (err != cudaSuccess) return err;
     for (long long i = 0; t + i * n < chunks; ++i) {

@@ -41,10 +41,10 @@ inline RowsOut rows2d(const double* a, long long nx, long long ny, long long nb,
 class StateIO {
  public:
   ~StateIO() { release(); }
-  // Both return cudaSuccess once the host array is complete (download) or the
-  // host array may change again (upload; the device side is complete too).
-  // Work already on the stream comes first.  Without page-locked memory both
-  // go through ordinary memory.
+  // A download returns once the host array is complete.  An uploaded array may
+  // change again, and the device side is complete, once the stream has been
+  // waited for, as after cudaMemcpyAsync.  Work already on the stream comes
+  // first.  Without page-locked memory both go through ordinary memory.
   cudaError_t download(const RowsOut& r, int device, cudaStream_t st);
   cudaError_t upload(void* dst, const void* src, size_t bytes, int device, cudaStream_t st);
   void release();

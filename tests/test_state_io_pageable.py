@@ -17,8 +17,10 @@ static int pins = 0;
 static cudaError_t no_pin(void**, size_t) { ++pins; return cudaErrorMemoryAllocation; }
 static cudaError_t copy(void* d, const void* s, size_t n, cudaMemcpyKind, cudaStream_t) { memcpy(d, s, n); return cudaSuccess; }
 static cudaError_t fine() { return cudaSuccess; }
+static cudaError_t attributes(cudaPointerAttributes* a, const void*) { a->type = cudaMemoryTypeUnregistered; return cudaSuccess; }
 #define cudaMallocHost no_pin
 #define cudaMemcpyAsync copy
+#define cudaPointerGetAttributes attributes
 #define cudaStreamSynchronize(st) fine()
 #define cudaSetDevice(d) fine()
 #define cudaGetLastError() fine()
@@ -99,6 +101,7 @@ static cudaError_t unpin(void* p) { free(p); return cudaSuccess; }
 static cudaError_t copy(void* d, const void* s, size_t n, cudaMemcpyKind, cudaStream_t) { memcpy(d, s, n); return cudaSuccess; }
 static cudaError_t event(cudaEvent_t* e, unsigned) { *e = (cudaEvent_t)1; return cudaSuccess; }
 static cudaError_t fine() { return cudaSuccess; }
+static cudaError_t attributes(cudaPointerAttributes* a, const void*) { a->type = cudaMemoryTypeUnregistered; return cudaSuccess; }
 namespace std {
 struct no_thread {  // starts once, then finds no memory
   static inline int made = 0;
@@ -115,6 +118,7 @@ struct no_thread {  // starts once, then finds no memory
 #define cudaMallocHost pin
 #define cudaFreeHost unpin
 #define cudaMemcpyAsync copy
+#define cudaPointerGetAttributes attributes
 #define cudaEventCreateWithFlags event
 #define cudaEventDestroy(e) fine()
 #define cudaEventRecord(e, st) fine()

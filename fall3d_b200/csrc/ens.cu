@@ -547,6 +547,7 @@ extern "C" int f3d_ens_set_class_grid(f3d_ens* e, int ci, const double* dX1_p, c
   if (!dX1_p || !dX1_b || !dX2_p || !dX2_b || !dX3_p || !dX3_b || !Hm1_p || !Hm2_p || !Hm3_p)
     return set_error_msg("f3d_ens_set_class_grid: null array");
   ECK(cudaSetDevice(e->device));
+  ECK(cudaStreamSynchronize(e->st));  // the copies below do not wait for steps in flight
   EnsClass& k = e->cls[ci];
   const size_t nx = k.nx, ny = k.ny, nz = k.nz;
   const double* src[6] = {dX1_p, dX1_b, dX2_p, dX2_b, dX3_p, dX3_b};
@@ -667,6 +668,7 @@ extern "C" int f3d_ens_set_class_terrain(f3d_ens* e, int ci, int map_v, double X
   if (map_v != 0 && (!X3_c || !X3_p || !dhdx_p || !dhdy_p || !(X3max > 0.0)))
     return set_error_msg("f3d_ens_set_class_terrain: sigma mappings need X3max > 0, X3_c, X3_p and the slopes");
   ECK(cudaSetDevice(e->device));
+  ECK(cudaStreamSynchronize(e->st));  // the copies below do not wait for steps in flight
   EnsClass& k = e->cls[ci];
   const size_t nx = k.nx, ny = k.ny, nz = k.nz;
   if (!k.terrain && ealloc(e, &k.terrain, (nz + 1) + nz + 2 * nx * ny)) return 1;
@@ -868,6 +870,7 @@ extern "C" int f3d_ens_set_member_source(f3d_ens* e, int mi, int n, const int* i
   const EnsClass& k = e->cls[e->member_class[mi]];
   if (!k.grid_set) return set_error_msg("f3d_ens_set_member_source: grid not set");
   ECK(cudaSetDevice(e->device));
+  ECK(cudaStreamSynchronize(e->st));  // the copies below do not wait for steps in flight
   MemberDev& m = e->hm[mi];
   std::vector<int> cell(n);
   std::vector<double> vol(n);
@@ -902,6 +905,7 @@ extern "C" int f3d_ens_upload_member_state(f3d_ens* e, int mi, const double* my_
                                            const double* my_acum) {
   if (!e || mi < 0 || mi >= e->nm) return set_error_msg("f3d_ens_upload_member_state: bad member");
   ECK(cudaSetDevice(e->device));
+  ECK(cudaStreamSynchronize(e->st));  // the copies below do not wait for steps in flight
   const EnsClass& k = e->cls[e->member_class[mi]];
   MemberDev& m = e->hm[mi];
   const size_t nx = k.nx, ny = k.ny, nz = k.nz, nb = e->nb;
@@ -1459,6 +1463,7 @@ extern "C" int f3d_ens_set_member_gravity_current(f3d_ens* e, int mi, const doub
     memcpy(h + o_lat_p, lat_p, k.ny * 8);
     memcpy(h + o_hm1_c, Hm1_c, (k.ny + 1) * 8);
     if (!k.gc_xy && ealloc(e, &k.gc_xy, n)) return 1;
+    ECK(cudaStreamSynchronize(e->st));  // steps in flight read the old ones
     ECK(cudaMemcpy(k.gc_xy, h, n * 8, cudaMemcpyHostToDevice));
   } else if (k.gc_host.size() != n) {
     return set_error_msg("f3d_ens_set_member_gravity_current: the class's coordinates not given");
@@ -1733,6 +1738,7 @@ extern "C" int f3d_ens_set_class_wet_deposition(f3d_ens* e, int ci, double a, do
   if (!k.grid_set) return set_error_msg("f3d_ens_set_class_wet_deposition: class grid not set");
   if (e->nb > 64) return set_error_msg("f3d_ens_set_class_wet_deposition: at most 64 bins");
   ECK(cudaSetDevice(e->device));
+  ECK(cudaStreamSynchronize(e->st));  // the copies below do not wait for steps in flight
   std::vector<double> powpb;
   std::vector<int> ktop;
   if (!wet_tables(k.nx, k.ny, k.nz, b, pre, pblh, h_c, z_c, powpb, ktop))
@@ -1825,6 +1831,7 @@ extern "C" int f3d_ens_set_class_corner_heights(f3d_ens* e, int ci, const double
   ECK(cudaSetDevice(e->device));
   const size_t n = (size_t)(k.nx + 1) * (k.ny + 1) * (k.nz + 1);
   if (!k.zc && ealloc(e, &k.zc, n)) return 1;
+  ECK(cudaStreamSynchronize(e->st));  // steps in flight read the old ones
   ECK(cudaMemcpy(k.zc, z_c, n * 8, cudaMemcpyHostToDevice));
   return 0;
 }

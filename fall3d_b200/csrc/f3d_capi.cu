@@ -448,6 +448,7 @@ extern "C" int f3d_ads_set_grid(f3d_ctx* c, const double* dX1_p, const double* d
   if (!dX1_p || !dX1_b || !dX2_p || !dX2_b || !dX3_p || !dX3_b || !Hm1_p || !Hm2_p || !Hm3_p)
     return set_err("f3d_ads_set_grid: null array");
   CK(cudaSetDevice(c->device));
+  CK(cudaStreamSynchronize(c->st));  // the copies below do not wait for steps in flight
   MemberDev& m = c->hm;
   const size_t nx = c->nx, ny = c->ny, nz = c->nz;
   if (h2d(c, (void*)m.dx1p, dX1_p, (nx + 4) * 8) || h2d(c, (void*)m.dx1b, dX1_b, (nx + 3) * 8) ||
@@ -571,6 +572,7 @@ extern "C" int f3d_ads_set_terrain(f3d_ctx* c, int map_v, double X3max, const do
   if (map_v != 0 && (!X3_c || !X3_p || !dhdx_p || !dhdy_p || !(X3max > 0.0)))
     return set_err("f3d_ads_set_terrain: sigma mappings need X3max > 0, X3_c, X3_p and the slopes");
   CK(cudaSetDevice(c->device));
+  CK(cudaStreamSynchronize(c->st));  // the copies below do not wait for steps in flight
   const size_t nx = c->nx, ny = c->ny, nz = c->nz;
   if (!c->d_terrain && dalloc(c, &c->d_terrain, (nz + 1) + nz + 2 * nx * ny)) return 1;
   if (map_v != 0) {
@@ -813,6 +815,7 @@ extern "C" int f3d_ads_set_wet_deposition(f3d_ctx* c, double a, double b, const 
   if (!c->grid_set) return set_err("f3d_ads_set_wet_deposition: grid not set");
   if (c->nb > 64) return set_err("f3d_ads_set_wet_deposition: at most 64 bins");
   CK(cudaSetDevice(c->device));
+  CK(cudaStreamSynchronize(c->st));  // the copies below do not wait for steps in flight
   const size_t ncol = (size_t)c->nx * c->ny;
   std::vector<double> powpb;
   std::vector<int> ktop;
@@ -958,6 +961,7 @@ extern "C" int f3d_ads_set_gravity_current(f3d_ctx* c, const double params[11], 
     memcpy(h + o_lat_p, lat_p, c->ny * 8);
     memcpy(h + o_hm1_c, Hm1_c, (c->ny + 1) * 8);
     if (!c->d_gc_xy && dalloc(c, &c->d_gc_xy, n)) return 1;
+    CK(cudaStreamSynchronize(c->st));  // steps in flight read the old ones
     CK(cudaMemcpy(c->d_gc_xy, h, n * 8, cudaMemcpyHostToDevice));
   } else if (c->gc_host.size() != n) {
     return set_err("f3d_ads_set_gravity_current: coordinates not given");
@@ -1008,6 +1012,7 @@ extern "C" int f3d_ads_set_corner_heights(f3d_ctx* c, const double* z_c) {
   CK(cudaSetDevice(c->device));
   const size_t n = (size_t)(c->nx + 1) * (c->ny + 1) * (c->nz + 1);
   if (!c->d_zc && dalloc(c, &c->d_zc, n)) return 1;
+  CK(cudaStreamSynchronize(c->st));  // steps in flight read the old ones
   CK(cudaMemcpy(c->d_zc, z_c, n * 8, cudaMemcpyHostToDevice));
   return 0;
 }
@@ -1133,6 +1138,7 @@ extern "C" int f3d_ads_set_source_dense(f3d_ctx* c, const double* my_s) {
 extern "C" int f3d_ads_upload_state(f3d_ctx* c, const double* my_c, const double* my_acum) {
   if (!c) return set_err("f3d_ads_upload_state: null context");
   CK(cudaSetDevice(c->device));
+  CK(cudaStreamSynchronize(c->st));  // the copies below do not wait for steps in flight
   MemberDev& m = c->hm;
   const size_t nx = c->nx, ny = c->ny, nz = c->nz, nb = c->nb;
   if (my_c) {

@@ -268,10 +268,14 @@ struct RangeArgs {
 // Host: bins per sweep block (its four warps take that many bins of one tile
 // of 32 pencils, or as many more tiles).  Bins of a tile share its face data
 // in L1, but a bin group that nb does not fill leaves warps idle that the
-// block's registers pay for: 4, 2 or 1, the largest that divides nb.  Nine
-// bins by ones instead of fours: 0.36 to 0.27 ms a step (FP32, 201 x 147 x 43
-// full of ash), 0.47 to 0.40 (compensated); six by twos: z of 100 x 80 x 40 in
-// FP64 166 to 108 us; eight by ones instead of fours would cost 24%.
+// block's registers pay for: 4, 2 or 1, the largest that divides nb.  A step of
+// 201 x 147 x 43 cells full of ash with 1, 2 and 4 bins a block, us:
+//   bins                7               9              11              14              15
+//   compensated  337  351  350   444  450  531   477  524  559   608  603  663   634  650  673
+//   FP64        2026 2108 2076  2449 2599 3119  2820 3142 3184  3638 3634 3733  3762 3780 3751
+// (FP32 goes with the compensated form; the most the rule loses is 2%, FP64 100
+// x 80 x 40 x 15).  Eight bins by ones instead of fours would cost 24%.  The
+// boundary fluxes are sums over the blocks, so their last bits go with it.
 inline int bins_per_block(int nb) { return nb % 4 == 0 ? 4 : nb % 2 == 0 ? 2 : 1; }
 
 // Correctly rounded a/b for a divisor with precomputed y = RN(1/b)
@@ -353,11 +357,12 @@ inline double div_small(double most) { return most <= 0x1p50 ? 0x1p-966 : 0x1p-9
 
 // A cell's diffusive flux P0 = n / dxp and right-hand side (P0 - P1) / dxb -
 // dF / dxb where one of the three numerators is small: one call for the three
-// divisions.  With a call for each the steps of wide plumes, whose fringe is
-// full of such values, took up to a fifth longer than with div_rn_recip
-// everywhere (y of 301 x 227 x 37 x 4: 1.15 to 1.51 ms; 1.23 with the one
-// call, later scaled and less often needed); inline in each place it costs 255
-// registers and 7 minutes of compiling for no gain.
+// divisions.  The fringe of a wide plume is full of such values; a step of
+// 301 x 227 x 37 x 4 cells takes 3.66 ms there (4.31 with a call for each
+// division, 3.53 with div_rn_recip everywhere) and 1.97 without a fringe (2.50
+// with div_rn_recip).  Inline in each place it costs 255 registers and 7
+// minutes of compiling for no gain; a warp-wide mode that follows the last
+// block's values makes every sweep 10% slower.
 static __device__ __noinline__ double2 rhs_small(double n, double P1, double dF, double dxp, double rdxp, double dxb,
                                                  double rdxb) {
   // the scaled quotients stay below 2^1001

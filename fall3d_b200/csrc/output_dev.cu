@@ -43,7 +43,7 @@ __device__ __forceinline__ double cs_interior(const OutArgs& a, int b, int i, in
 
 // The interior cs of the selected bins, once per mass point (every value is
 // read by the eight corners around it).  A block takes rows of x, so that the
-// metric of a row is formed once per point and no 64-bit division is left.
+// 64-bit divisions that find its place are taken once a row.
 __global__ void k_out_cs(OutArgs a, int nsel) {
   const long long rows = (long long)a.ny * a.nz * nsel;
   for (long long r = blockIdx.x; r < rows; r += gridDim.x) {

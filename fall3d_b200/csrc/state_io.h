@@ -53,11 +53,11 @@ class StateIO {
   static constexpr int kSlots = 8;  // two per host thread
   // Eight slots of 192 KB come with the 2 MB that the driver page-locks for
   // the context's first small allocation, so that the first transfer of a
-  // context takes no longer than the later ones.  Slots of 1 MB cost 5-10 ms
-  // to page-lock and save 2.5 ms per 100 MB, so they are taken once a context
-  // has moved 384 MB.
-  static constexpr size_t kSlotBytes = 192 << 10, kLargeSlotBytes = 1 << 20;
-  static constexpr size_t kLargeFrom = 384 << 20;
+  // context takes no longer than the later ones.  Slots of 512 KB take 5 ms to
+  // page-lock and save 2-3 ms per 100 MB (1 MB: 9 ms, no faster), so they are
+  // taken once a context has moved 128 MB.
+  static constexpr size_t kSlotBytes = 192 << 10, kLargeSlotBytes = 512 << 10;
+  static constexpr size_t kLargeFrom = 128 << 20;
   cudaError_t reserve(size_t total, size_t unit);
   char* pin_ = nullptr;
   size_t slot_bytes_ = 0;

@@ -22,7 +22,7 @@ def test_many_read_backs(built_lib, prec):
     with Domain(wl.grid, nb, precision=prec) as dom:
         dom.upload_state(c0, None)
         c = np.empty_like(c0)
-        for _ in range(21):  # 384 MB pass during the last ones
+        for _ in range(21):  # past the 128 MB that bring them
             c.fill(-7.0)
             dom.download_state(c, None)
             assert np.array_equal(c[2:-2, 2:-2, 2:-2], x)

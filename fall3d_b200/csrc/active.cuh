@@ -179,24 +179,13 @@ __global__ void __launch_bounds__(256) k_ranges32(const MemberDev* __restrict__ 
     }
   }
   __syncthreads();
-  // the lengths of all items for the host (box_gate.h), by the last block
-  if (threadIdx.x != 0) return;
-  for (int e = 0; e < 3; ++e)
-    if (sum[e]) {
-      atomicMax(a.acc + e, most[e]);
-      atomicAdd(a.acc + 3 + e, sum[e]);
-    }
-  __threadfence();
-  if (atomicAdd(a.acc + 6, 1u) != gridDim.x - 1) return;
-  __threadfence();
-  volatile unsigned int* pub = a.pub;
-  for (int e = 0; e < 6; ++e) pub[1 + e] = atomicExch(a.acc + e, 0u);
-  pub[7] = (unsigned int)a.dirs;
-  a.acc[6] = 0u;
-  const unsigned int run = a.acc[7] + 1u;
-  a.acc[7] = run;
-  __threadfence_system();
-  pub[0] = run;
+  // the lengths of all items for the host (box_gate.h); k_flux_reduce passes
+  // them on at the end of the step, beside work that takes longer (here, with
+  // a ticket and a write to the host, they cost 6 us a step)
+  if (threadIdx.x < 3 && sum[threadIdx.x]) {
+    atomicMax(a.acc + threadIdx.x, most[threadIdx.x]);
+    atomicAdd(a.acc + 3 + threadIdx.x, sum[threadIdx.x]);
+  }
 }
 
 }  // namespace f3d

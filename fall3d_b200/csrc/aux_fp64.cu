@@ -335,16 +335,31 @@ void launch_set_dt_stime(MemberDev* members, int mi, double dt, double stime, cu
 // Kahan-compensated update.
 // A block per member and direction: one after the other they took 24 us on a
 // 400 x 300 x 60 x 8 step, a block's chain of loads each (14 us side by side).
-__global__ void k_flux_reduce(const MemberDev* __restrict__ members, int dirmask) {
+// One more block passes the lengths of the step's ranges on to the host.
+__global__ void k_flux_reduce(const MemberDev* __restrict__ members, int dirmask, GatePub g) {
   __shared__ double sa[256], sb[256];
+  if (blockIdx.y == 3) {
+    if (blockIdx.x != 0 || threadIdx.x != 0) return;
+    volatile unsigned int* pub = g.pub;
+    for (int e = 0; e < 6; ++e) {
+      pub[1 + e] = g.acc[e];
+      g.acc[e] = 0u;
+    }
+    pub[7] = (unsigned int)g.dirs;
+    const unsigned int run = g.acc[7] + 1u;
+    g.acc[7] = run;
+    __threadfence_system();
+    pub[0] = run;
+    return;
+  }
   member_flux_reduce(members[blockIdx.x], dirmask & 1 << blockIdx.y, sa, sb);
 }
 __global__ void k_zero_step(const MemberDev* __restrict__ members) {
   const MemberDev& m = members[blockIdx.x];
   if (threadIdx.x < 6) m.flux_step[threadIdx.x] = 0.0;
 }
-void launch_flux_reduce(const MemberDev* members, int nmembers, int dirmask, cudaStream_t st) {
-  k_flux_reduce<<<dim3(nmembers, 3), 256, 0, st>>>(members, dirmask);
+void launch_flux_reduce(const MemberDev* members, int nmembers, int dirmask, const GatePub& g, cudaStream_t st) {
+  k_flux_reduce<<<dim3(nmembers, g.pub ? 4 : 3), 256, 0, st>>>(members, dirmask, g);
 }
 void launch_zero_step(const MemberDev* members, int nmembers, cudaStream_t st) {
   k_zero_step<<<nmembers, 32, 0, st>>>(members);

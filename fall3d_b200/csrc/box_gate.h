@@ -3,10 +3,10 @@
 //
 // Finding the boxes costs two launches and a pass over the state, and pays
 // when it shortens the march.  How long a march is depends on the state, which
-// the host does not read; so the range kernel leaves the lengths of the last
-// step it ran for in page-locked memory, and the host looks there, without
-// waiting, when it puts the next step together.  Either way the step has the
-// same result, so a value that is some steps old costs time at most.
+// the host does not read; so a step with ranges leaves their lengths in
+// page-locked memory, and the host looks there, without waiting, when it puts
+// the next step together.  Either way the step has the same result, so a value
+// that is some steps old costs time at most.
 //
 // Looking for the boxes in every step, whatever they gained, made a step of
 // 48 x 40 x 24 x 4 cells 71 to 86 us, one of 157 x 93 x 37 x 8 full of ash 181
@@ -19,8 +19,8 @@
 
 namespace f3d {
 
-// What k_ranges32 leaves: a count of its runs, written last; the longest
-// range and the sum of all ranges per direction; the directions it ran for.
+// What such a step leaves: a count of them, written last; the longest range
+// and the sum of all ranges per direction; the directions it ran for.
 constexpr int kGateWords = 8;
 
 class BoxGate {
@@ -30,7 +30,8 @@ class BoxGate {
   void attach(const unsigned int* pub, bool compensated) {
     pub_ = pub;
     slower_ = compensated ? 1.12 : 1.05;
-    operator_cost_ = compensated ? 50.0 : 80.0;
+    step_cost_ = compensated ? 22.0 : 30.0;
+    operator_cost_ = compensated ? 55.0 : 100.0;
   }
   // The state was replaced (nothing in flight): start over.
   void reset() {
@@ -63,22 +64,28 @@ class BoxGate {
   }
 
  private:
-  // Cells marched in series: a block's own, or the blocks of an SM's slots
-  // one after the other (four of them on each of 148 SMs).
+  // How long a march is, in cells of a full device: 592 blocks are resident
+  // (four on each of 148 SMs), and where that is a round or less, the longest
+  // block's cells take 0.64 of a full device's time each, and the others' work
+  // the rest (a compensated step marches a cell in 0.42 us with few blocks, in
+  // 0.66 with all).
   static double length(int dirs, const int longest[3], const long long total[3]) {
     double s = 0.0;
-    for (int d = 0; d < 3; ++d)
-      if (dirs >> d & 1) s += std::max((double)longest[d], (double)total[d] / 592.0);
+    for (int d = 0; d < 3; ++d) {
+      const double all = (double)total[d] / 592.0;
+      if (dirs >> d & 1) s += std::max(0.64 * longest[d] + 0.36 * all, all);
+    }
     return s;
   }
-  // The two launches in cells marched: a step has them behind other work (14
-  // us; a compensated step marches a cell in 0.4-0.6 us, an FP32 one in 0.3),
-  // a lone operator waits for them (about 20 us).  A march over a range takes
-  // longer per cell than one over the pencil, whose ends the compiler knows
-  // to be the domain's (400 x 300 x 60 x 4 full of ash, compensated: 0.88 ms
-  // a step with ranges, 0.78 without; FP32 0.56 and 0.55).
-  double cost(int dirs) const { return (dirs & (dirs - 1)) ? 30.0 : operator_cost_; }
-  double slower_ = 1.12, operator_cost_ = 50.0;
+  // The two launches in such cells: a step has them behind other work (14 us;
+  // a cell takes 0.66 us compensated, 0.47 in FP32), a lone operator waits for
+  // them (20 us and more: y of 200 x 150 x 40 x 8 in FP32, a plume, 83 us
+  // without and 98 with).  A march over a range takes longer per cell than one
+  // over the pencil, whose ends the compiler knows to be the domain's (400 x
+  // 300 x 60 x 4 full of ash, compensated: 0.88 ms a step with ranges, 0.78
+  // without; FP32 0.56 and 0.55).
+  double cost(int dirs) const { return (dirs & (dirs - 1)) ? step_cost_ : operator_cost_; }
+  double slower_ = 1.12, step_cost_ = 22.0, operator_cost_ = 55.0;
   static constexpr int kLook = 32;  // steps between two looks at a state that boxes do not help
   struct Way {
     bool pays = true;

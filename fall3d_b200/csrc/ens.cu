@@ -37,7 +37,7 @@ void launch_source64(const MemberDev* members, int nmembers, cudaStream_t st);
 void launch_source32(const MemberDev* members, int nmembers, cudaStream_t st);
 void launch_conv(int which, const double* in, double* out, int nx, int ny, int nz, int nb,
                  cudaStream_t st);
-void launch_flux_reduce(const MemberDev* members, int nmembers, int dirmask, cudaStream_t st);
+void launch_flux_reduce(const MemberDev* members, int nmembers, int dirmask, const GatePub& g, cudaStream_t st);
 void launch_cfl(const MemberDev* members, int mi, double s, int criterion, double* out3,
                 cudaStream_t st, const GcArgs* gc = nullptr);
 void launch_mass(const MemberDev* members, int mi, int nb, int fp32, double* partials, int nblk,
@@ -1265,7 +1265,6 @@ int enqueue_step(f3d_ens* e, bool xfirst, bool boxes, bool advance, cudaEvent_t*
     a.grown[DIR_Y] = xfirst ? 1 << DIR_X : 0;
     a.grown[DIR_Z] = 1 << DIR_X | 1 << DIR_Y;
     a.acc = e->d_gate;
-    a.pub = e->h_gate;
     launch_ranges32(e->dm, e->nm, e->maxlev, a, e->st);
   }
   e->launches += (e->prec == F3D_PREC_FP64) ? 2 : boxes ? 3 : 1;
@@ -1281,7 +1280,7 @@ int enqueue_step(f3d_ens* e, bool xfirst, bool boxes, bool advance, cudaEvent_t*
     e->launches += 1;
     if (ev) ECK(cudaEventRecord(ev[2 + q], e->st));
   }
-  launch_flux_reduce(e->dm, e->nm, 7, e->st);
+  launch_flux_reduce(e->dm, e->nm, 7, boxes ? GatePub{e->d_gate, e->h_gate, 7} : GatePub{nullptr, nullptr, 0}, e->st);
   e->launches += 1;
   if (enqueue_wet_radio(e)) return 1;
   if (advance) {

@@ -32,7 +32,7 @@ void launch_conv(int which, const double* in, double* out, int nx, int ny, int n
 void launch_set_step(MemberDev* members, int mi, double dt, double time, int iiter,
                      cudaStream_t st);
 void launch_set_dt_stime(MemberDev* members, int mi, double dt, double stime, cudaStream_t st);
-void launch_flux_reduce(const MemberDev* members, int nmembers, int dirmask, cudaStream_t st);
+void launch_flux_reduce(const MemberDev* members, int nmembers, int dirmask, const GatePub& g, cudaStream_t st);
 void launch_zero_step(const MemberDev* members, int nmembers, cudaStream_t st);
 void launch_cfl(const MemberDev* members, int mi, double s, int criterion, double* out3,
                 cudaStream_t st, const GcArgs* gc = nullptr);
@@ -1217,11 +1217,14 @@ static int enqueue_ranges(f3d_ctx* c, int dirs, bool xfirst, bool* on) {
   a.grown[DIR_Y] = dirs & (xfirst ? 1 << DIR_X : 0);
   a.grown[DIR_Z] = dirs & (1 << DIR_X | 1 << DIR_Y);
   a.acc = c->d_gate;
-  a.pub = c->h_gate;
   launch_ranges32(c->dm, 1, c->nb * c->nz, a, c->st);
   c->launches += 2;
   CKL();
   return 0;
+}
+
+static GatePub gate_pub(const f3d_ctx* c, bool boxes, int dirs) {
+  return boxes ? GatePub{c->d_gate, c->h_gate, dirs} : GatePub{nullptr, nullptr, 0};
 }
 
 static int enqueue_sweep(f3d_ctx* c, int dir, bool boxes) {
@@ -1405,7 +1408,7 @@ static int enqueue_step(f3d_ctx* c, double dt, double time, int iiter) {
   rec(3);
   if (enqueue_sweep(c, DIR_Z, boxes)) return 1;
   rec(4);
-  launch_flux_reduce(c->dm, 1, 7, c->st);
+  launch_flux_reduce(c->dm, 1, 7, gate_pub(c, boxes, 7), c->st);
   c->launches += 1;
   CKL();
   if (enqueue_wet_radio(c, dt)) return 1;
@@ -1506,7 +1509,7 @@ static int solve_dir(f3d_ctx* c, int dir, double dt, double* a, double* b, const
   CK(cudaSetDevice(c->device));
   bool boxes;
   if (enqueue_ranges(c, 1 << dir, true, &boxes) || enqueue_sweep(c, dir, boxes)) return 1;
-  launch_flux_reduce(c->dm, 1, 1 << dir, c->st);
+  launch_flux_reduce(c->dm, 1, 1 << dir, gate_pub(c, boxes, 1 << dir), c->st);
   CKL();
   CK(cudaMemcpyAsync(c->h_pin, c->hm.flux_step, 6 * sizeof(double), cudaMemcpyDeviceToHost, c->st));
   CK(cudaStreamSynchronize(c->st));

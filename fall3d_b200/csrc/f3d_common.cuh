@@ -261,8 +261,14 @@ struct RangeArgs {
   int2* range[3];
   int nwork[3], grown[3];
   int dirs, bpb;
-  unsigned int* acc;  // [kGateWords] in device memory, zero between runs but for the last (box_gate.h)
-  unsigned int* pub;  // [kGateWords] page-locked: what the host reads
+  unsigned int* acc;  // BoxGate's words in device memory
+};
+// What k_flux_reduce passes on to the host after a step with ranges over dirs
+// (box_gate.h); null otherwise.
+struct GatePub {
+  unsigned int* acc;  // zero between steps but for the last word, the count of runs
+  unsigned int* pub;  // page-locked
+  int dirs;
 };
 
 // Host: bins per sweep block (its four warps take that many bins of one tile

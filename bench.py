@@ -365,32 +365,52 @@ def run_c2(args, ws, rank, local, pg):
             np.linalg.norm(b[..., q] - a[..., q]) / max(np.linalg.norm(a[..., q]), 1e-300)
             for q in range(a.shape[-1])))
         del c32
-    # ---- per-kernel profile (event-timed phases) for the roofline
-    dom.set_profiling(True)
-    t = t_end
-    for it in range(3):
-        dom.step_async(dt32, t, K + Wu + it)
-        t += dt32
-    prof, n = dom.get_profile()
-    dom.set_profiling(False)
-    per = {"x": prof[1] / n, "y": prof[2] / n, "z": prof[3] / n}
-    dom_k = max(per, key=per.get)
-    # the compensated form also reads and writes the low part (4 B each)
-    byts = sweep_bytes(wl, 4, dom_k) + (2.0 * 4 * cbs if prec == 2 else 0.0)
-    peak, kind = hbm_peak()
-    achieved = byts / (per[dom_k] / 1e3) / 1e9
-    out["roofline"] = {"bound": "hbm",
-                       "kernel": f"k_sweep32<{'xyz'.index(dom_k)},2,2,{int(prec == 2)}> ({dom_k} sweep)",
-                       "achieved": round(achieved, 1), "peak": peak, "unit": "GB/s",
-                       "frac": round(achieved / peak, 4), "peak_kind": kind,
-                       "traffic": load_traffic(f"sweep32{'c' if prec == 2 else ''}_{dom_k}", "c2"),
-                       "algorithmic_bytes": byts, "launch_ms": round(per[dom_k], 4),
-                       "sweep_ms": {k: round(v, 4) for k, v in per.items()}}
     # ---- e2e through the C ABI with host buffers
     out["e2e"] = e2e_c2(dom, wl, dt32, K, local, pg, ws, cbs)
+    out["full_state"], out["roofline"] = full_state(dom, wl, dt32, prec, K, local, pg, ws)
     dom.close()
     out["workload"] = wl
     return out
+
+
+def full_state(dom, wl, dt, prec, K, device, pg, ws):
+    """Rate and dominant kernel of a domain with ash in every cell.  The
+    sweeps of the precision forms leave out cells without any, so a run that
+    starts from rest says nothing about bytes per second: its cells are mostly
+    not touched.  Here all of them are."""
+    g, nb = wl.grid, wl.nbins
+    rng = np.random.default_rng(7)
+    c = np.zeros((nb, g.nz + 4, g.ny + 4, g.nx + 4))
+    for b in range(nb):
+        c[b, 2:-2, 2:-2, 2:-2] = rng.uniform(1e-6, 1e-3, (g.nz, g.ny, g.nx))
+    dom.upload_state(c.T, None)
+    del c
+    f = np.zeros(6)
+    for it in range(4):  # one by one: the library sees that boxes do not pay here
+        dom.F3D_time_step(dt, 0.0, it, f)
+    ms, _, t = time_steps(dom, dt, K, 2, device, pg)
+    ms = max_over_ranks(pg, ms) / K
+    dom.set_profiling(True)
+    for it in range(4):
+        dom.step_async(dt, t, it)
+    prof, n = dom.get_profile()
+    dom.set_profiling(False)
+    per = {"x": prof[1] / n, "y": prof[2] / n, "z": prof[3] / n}
+    dk = max(per, key=per.get)
+    # the compensated form also reads and writes the low part (4 B each)
+    cells = float(g.nx * g.ny * g.nz * nb)
+    byts = sweep_bytes(wl, 4, dk) + (2.0 * 4 * cells if prec == 2 else 0.0)
+    peak, kind = hbm_peak()
+    achieved = byts / (per[dk] / 1e3) / 1e9
+    tkey = f"sweep32{'c' if prec == 2 else ''}_{dk}"
+    what = f"one {g.nx}x{g.ny}x{g.nz} domain, {nb} bins, ash in every cell"
+    return ({"value": ws * cells / (ms / 1e3), "unit": UNIT, "ms_per_step": round(ms, 4), "workload": what},
+            {"bound": "hbm", "kernel": f"k_sweep32<{'xyz'.index(dk)},2,2,{int(prec == 2)}> ({dk} sweep; {what})",
+             "achieved": round(achieved, 1), "peak": peak, "unit": "GB/s",
+             "frac": round(achieved / peak, 4), "peak_kind": kind,
+             "traffic": load_traffic(tkey, "full_state", byts), "algorithmic_bytes": byts,
+             "traffic_source": traffic_source(tkey, "full_state"),
+             "launch_ms": round(per[dk], 4), "sweep_ms": {k: round(v, 4) for k, v in per.items()}})
 
 
 def e2e_c2(dom, wl, dt, K, device, pg, ws, cbs):
@@ -630,6 +650,7 @@ def run_ensemble(args, ws, rank, local, pg):
         i64, i32 = c64[2:-2, 2:-2, 2:-2, :], c32[2:-2, 2:-2, 2:-2, :]
         d64, d32 = deposit_mass(g, a64), deposit_mass(g, a32)
         errs.append({"member": m, "grid": f"{g.nx}x{g.ny}x{g.nz}",
+                     "cells_with_ash": float(np.count_nonzero(i32) / i32.size),
                      "conc_rel_l2": float(np.linalg.norm(i32 - i64) / np.linalg.norm(i64)),
                      "conc_rel_l2_worst_bin": float(max(np.linalg.norm(i32[..., q] - i64[..., q]) /
                                                         max(np.linalg.norm(i64[..., q]), 1e-300)
@@ -656,10 +677,10 @@ def run_ensemble(args, ws, rank, local, pg):
 
 
 # FP64 operations (DFMA + DADD + DMUL, thread level) per cell*bin*step of the
-# plain FP64 sweeps, from ncu on the 400x300x60x20 case
+# plain FP64 sweeps from rest, from ncu on the 200x150x40 case with 8 bins
 # (profiles/k_sweep64_c2.md); FP64 pipe of the B200: 64 operations per clock
 # per SM on 148 SMs.
-FP64_OPS_PER_CELLBIN_STEP = 1066
+FP64_OPS_PER_CELLBIN_STEP = 708
 
 
 def fp64_roofline(steps_value, sm_mhz):
@@ -704,52 +725,29 @@ def time_plain_fp32(args, ew, ws, local, pg, tuning):
             "note": "plain FP32 state, same workload and tuning, step kernels only"}
 
 
-def ens_roofline(r, K):
-    """Dominant kernel of the ensemble step, from event-timed profiled steps
-    in the tuned mode; algorithmic bytes: every member's concentration (the
-    compensated form: its hi and lo parts) read and written once per sweep,
-    the class fields (shared by the members of a class) once."""
-    ens, ew = r["ens"], r["workload"]
+def ens_phases(r):
+    """Event-timed phases of profiled steps in the tuned mode, as they follow
+    the timed ones (a persistent step is one kernel: "x").  "prep" holds the
+    source and the search for the cells with ash."""
+    ens = r["ens"]
     ens.set_profiling(True)
     ens.run(3)
     ens.synchronize()
     ms, n = ens.get_profile()
     ens.set_profiling(False)
-    per = ms / max(n, 1)
-    nb = ew.nbins
+    return {k: round(float(v) / max(n, 1), 3) for k, v in zip(("prep", "x", "y", "z", "flux"), ms)}
 
-    def bytes_dir(d):
-        tot = 0.0
-        for ci, wl in enumerate(ew.classes):
-            g = wl.grid
-            nmem = ew.member_class.count(ci)
-            cells = g.nx * g.ny * g.nz
-            # c read + write: FP32 (4 B), or the compensated pair hi + lo (8 B)
-            tot += nmem * 2.0 * r["state_bytes"] * cells * nb
-            tot += sweep_bytes(wl, 4, d) - 2.0 * 4 * cells * nb  # class fields once
-        return tot
 
-    peak, kind = hbm_peak()
-    if r["tuning"]["mode"] == "persistent":
-        byts = sum(bytes_dir(d) for d in "xyz")
-        t = per[1]
-        name = "k_fused32 (persistent step: x, y, z sweeps of all 64 members)"
-        tkey = "fused32"
-    else:
-        sw = {"x": per[1], "y": per[2], "z": per[3]}
-        dk = max(sw, key=sw.get)
-        byts = bytes_dir(dk)
-        t = sw[dk]
-        cmp = int(r["state_bytes"] == 8)
-        name = f"k_sweep32<{'xyz'.index(dk)},2,2,{cmp}> ({dk} sweep of all 64 members)"
-        tkey = f"sweep32{'c' if cmp else ''}_{dk}"
-    achieved = byts / (t / 1e3) / 1e9
-    return {"bound": "hbm", "kernel": name, "achieved": round(achieved, 1), "peak": peak, "unit": "GB/s",
-            "frac": round(achieved / peak, 4), "peak_kind": kind,
-            "traffic": load_traffic(tkey, "ensemble", byts), "algorithmic_bytes": byts,
-            "traffic_source": traffic_source(tkey, "ensemble"),
-            "launch_ms": round(t, 3),
-            "phase_ms": {k: round(float(v), 3) for k, v in zip(("prep", "x", "y", "z", "flux"), per)}}
+def ens_full_state(args, ew, dts, reps, local, pg, ws):
+    """full_state of the middle grid class."""
+    from fall3d_b200.ads import Domain
+    wl, prec = ew.classes[1], PRECISIONS[args.precision]
+    dom = Domain(wl.grid, wl.nbins, 2, 2, prec, device=local)
+    dom.set_meteo(wl.u12, wl.v12, wl.w12, wl.k1, wl.k2, wl.k3, None, wl.t_its, wl.t_ite)
+    dom.phys_get_vset(wl.vset_model, wl.rhoc, wl.tc, wl.diam, wl.rhop, wl.psi, wl.bin_cat)
+    out = full_state(dom, wl, float(dts[reps[1]]), prec, args.steps, local, pg, ws)
+    dom.close()
+    return out
 
 
 def pinned_copy(a):
@@ -902,7 +900,10 @@ def line_ensemble(args, ws, res):
         "steps_only_value": res["steps_only_value"],
         "gpu_launches": res["launches"],
         "clocks": res["clocks"],
-        "roofline": res["roofline"],
+        "phase_ms": res["phase_ms"],
+        # value counts every cell of the domains; this part of them held ash
+        # after the timed steps (first member of each grid class)
+        "cells_with_ash": [round(x["cells_with_ash"], 4) for x in e],
         "e2e": res["e2e"],
         "errors_vs_fp64": {
             "conc_rel_l2_max": max(x["conc_rel_l2"] for x in e),
@@ -947,7 +948,7 @@ def main():
         return
     if args.workload == "ensemble":
         res = run_ensemble(args, ws, rank, local, pg)
-        res["roofline"] = ens_roofline(res, args.steps)
+        res["phase_ms"] = ens_phases(res)
         res["e2e"] = e2e_ensemble(res, args.steps, pg, ws)
         if rank == 0:
             line = line_ensemble(args, ws, res)
@@ -958,6 +959,9 @@ def main():
         tuning = res["ens"].tuning
         res["ens"].close()
         res["sur"].close()
+        full = ens_full_state(args, res["workload"], res["dts"], res["reps"], local, pg, ws)
+        if rank == 0:
+            line["full_state"], line["roofline"] = full
         if args.precision == "fp32c" and not args.no_plain_fp32:
             plain = time_plain_fp32(args, res["workload"], ws, local, pg, tuning)
             if rank == 0:
@@ -987,6 +991,7 @@ def main():
             "speedup_vs_fp64": res["value"] / res["fp64_value"],
             "gpu_launches": res["launches"],
             "clocks": res["clocks"],
+            "full_state": res["full_state"],
             "roofline": res["roofline"],
             "e2e": res["e2e"],
         }

@@ -14,11 +14,10 @@
 //
 // The host asks for all this only where it pays (box_gate.h): a sweep without
 // ranges marches whole pencils.  An eruption's plume fills a small part of its
-// domain for most of a run.  On
-// the B200 the three compensated sweeps of a plume in 400 x 300 x 60 x 8 cells
-// went from 1.38 to 0.35 ms a step, with 0.08 ms for the boxes and ranges; with
-// ash everywhere (203 x 149 x 41 x 9) they went from 0.411 to 0.434 ms, with
-// 0.014 ms.  Measured against it and left: looking at the pencils from both
+// domain for most of a run.  On the B200 the three compensated sweeps of a
+// plume in 400 x 300 x 60 x 8 cells went from 1.38 to 0.35 ms a step, with 0.08
+// ms for the boxes and ranges (with ash everywhere they take 14 us and save
+// nothing).  Measured against it and left: looking at the pencils from both
 // ends in each sweep (0.50 ms on the plume, a memory latency ahead of every
 // short march) and testing every block of the march (0.56 ms; the dense plain
 // FP32 y and z sweeps 25% slower: registers).

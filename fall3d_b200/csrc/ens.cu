@@ -1060,7 +1060,7 @@ int fused_setup(f3d_ens* e, const void** func, int* smem) {
 
 // Enqueue one step.  set_host: dt/time come from the host arrays.
 // One step on the stream.  ev (profiling only, never while capturing):
-// ev[0] before the step, ev[1] after prep/source, ev[2 + q] after the q-th
+// ev[0] before the step, ev[1] after prep, source and boxes, ev[2 + q] after the q-th
 // sweep of the step's order, ev[5] at the end; in the persistent mode the
 // whole step lies between ev[0] and ev[5].
 // exp(-kn dt) of every radionuclide bin (and of its Sr90 parent) for each

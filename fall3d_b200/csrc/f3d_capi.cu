@@ -1373,7 +1373,7 @@ static int enqueue_wet_radio(f3d_ctx* c, double dt) {
 }
 
 static int enqueue_step(f3d_ctx* c, double dt, double time, int iiter) {
-  // event slots: 0 start, 1 after prep+source, 2..4 after the 1st/2nd/z sweep, 5 end
+  // event slots: 0 start, 1 after prep, source and the search for boxes, 2..4 after the 1st/2nd/z sweep, 5 end
   auto rec = [&](int k) { if (c->prof) cudaEventRecord(c->ev[k], c->st); };
   rec(0);
   // gravity current at this time; the precision form's sweeps are switched to

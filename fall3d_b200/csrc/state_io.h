@@ -53,10 +53,11 @@ class StateIO {
   static constexpr int kSlots = 8;  // two per host thread
   // Eight slots of 192 KB come with the 2 MB that the driver page-locks for
   // the context's first small allocation, so that the first transfer of a
-  // context takes no longer than the later ones.  Slots of 512 KB take 5 ms to
-  // page-lock and save 2-3 ms per 100 MB (1 MB: 9 ms, no faster), so they are
-  // taken once a context has moved 128 MB.
-  static constexpr size_t kSlotBytes = 192 << 10, kLargeSlotBytes = 512 << 10;
+  // context takes no longer than the later ones.  Slots of 1 MB take 5-9 ms to
+  // page-lock and save 2-3 ms per 100 MB (512 KB as much on the way out, but a
+  // 200 x 150 x 40 x 8 meteo update takes 19.1 ms with them against 17.7), so
+  // they are taken once a context has moved 128 MB.
+  static constexpr size_t kSlotBytes = 192 << 10, kLargeSlotBytes = 1 << 20;
   static constexpr size_t kLargeFrom = 128 << 20;
   cudaError_t reserve(size_t total, size_t unit);
   char* pin_ = nullptr;

@@ -270,7 +270,8 @@ int f3d_ads_get_stream(f3d_ctx *ctx, void **stream);
 
 /* Per-phase device timing with CUDA events on the context stream.  When on,
  * every step records events around its phases and waits for them; the
- * accumulated milliseconds are ms[0] prep+source, ms[1] x sweep, ms[2] y
+ * accumulated milliseconds are ms[0] prep+source (and, in the precision
+ * forms, the search for the cells with ash when there is one), ms[1] x sweep, ms[2] y
  * sweep, ms[3] z sweep, ms[4] flux reduction, ms[5] whole step. */
 int f3d_ads_set_profiling(f3d_ctx *ctx, int on);
 int f3d_ads_get_profile(f3d_ctx *ctx, double ms[6], int *nsteps);
@@ -543,8 +544,9 @@ int f3d_ens_output_member_species(f3d_ens *ens, int member, const int *bin_in,
                                   double *grn_load);
 /* Per-phase device timing: while on, f3d_ens_run enqueues steps without the
  * graph and records events between phases; ms[5] accumulates
- * {prep+source, x sweep, y sweep, z sweep, flux+clock} (persistent mode: the
- * fused step kernel in ms[1]) over nsteps steps.  Turning it on resets. */
+ * {prep+source and the search for the cells with ash, x sweep, y sweep, z
+ * sweep, flux+clock} (persistent mode: the fused step kernel in ms[1]) over
+ * nsteps steps.  Turning it on resets. */
 int f3d_ens_set_profiling(f3d_ens *ens, int on);
 int f3d_ens_get_profile(f3d_ens *ens, double *ms, int *nsteps);
 int f3d_ens_synchronize(f3d_ens *ens);
